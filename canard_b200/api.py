@@ -384,7 +384,8 @@ class Context:
             self._check(-k)
         kinds = {0: "fp64", 1: "fp32-split", 2: "fp64-tile/fp32-split", 3: "fp32-one-lane",
                  4: "fp64-tile/fp32-one-lane", 5: "fp64-tmem", 6: "fp64-stream/fp32-split", 7: "fp64-split",
-                 8: "fp64-quad", 9: "fp32-quad", 10: "fp64-twist", 11: "fp32-twist", 12: "fp64-tile/fp32-twist"}
+                 8: "fp64-quad", 9: "fp32-quad", 10: "fp64-twist", 11: "fp32-twist", 12: "fp64-tile/fp32-twist",
+                 13: "fp64-one-lane"}
         out = []
         for i in range(k):
             g, d, kd, nc, best, dflt = rep[6 * i:6 * i + 6]
@@ -395,13 +396,14 @@ class Context:
 
     LINE_KINDS = {"default": -1, "fp64": 0, "fp32-split": 1, "fp64-tile/fp32-split": 2, "fp32-one-lane": 3,
                   "fp64-tile/fp32-one-lane": 4, "fp64-tmem": 5, "fp64-stream/fp32-split": 6, "fp64-split": 7,
-                  "fp64-quad": 8, "fp32-quad": 9, "fp64-twist": 10, "fp32-twist": 11, "fp64-tile/fp32-twist": 12}
+                  "fp64-quad": 8, "fp32-quad": 9, "fp64-twist": 10, "fp32-twist": 11, "fp64-tile/fp32-twist": 12,
+                  "fp64-one-lane": 13}
 
     def set_line_kind(self, group, direction, kind, chunks=0):
         """Pins the line kernel of a group ("filter", "viscous", "flux") and
         direction ("xi", "eta", "zeta"), by name from LINE_KINDS; "fp64",
         "fp64-tmem" give results bit-identical to the reference's order,
-        "fp64-split" and "fp64-twist" (the fast FP64 mode's kinds) differ at
+        "fp64-split", "fp64-twist" and "fp64-one-lane" (the fast FP64 mode's kinds) differ at
         rounding level."""
         g = ("filter", "viscous", "flux").index(group)
         d = ("xi", "eta", "zeta").index(direction)

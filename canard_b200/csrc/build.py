@@ -18,7 +18,7 @@ BUILD = os.path.join(HERE, "_build")
 # (source, FMA contraction allowed)
 UNITS = [("canard.cu", False), ("kernels_f32.cu", True), ("host.cpp", False), ("restart.cpp", False),
          ("plt.cpp", False)]
-DEPS = [u for u, _ in UNITS] + ["kernels.cuh", "kernels_f32.h", "kernels_setup.cuh", "kernels_tm.cuh", "host.h"]
+DEPS = [u for u, _ in UNITS] + ["kernels.cuh", "kernels_line.cuh", "kernels_f32.h", "kernels_setup.cuh", "kernels_tm.cuh", "host.h"]
 
 
 def nvcc():

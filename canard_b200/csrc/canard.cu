@@ -95,8 +95,13 @@ enum LineKind {
   LK_F32_QUAD = 9,             // derivative: FP32 fields, four lanes per line
   LK_F64_TWIST = 10,           // FP64 fields, two-ended FP64 solve with FMA (two warps per 32 lines)
   LK_F32_TWIST = 11,           // derivative: FP32 fields, two-ended FP32 solve
-  LK_F64_TILE_F32_TWIST = 12   // filter: FP64 field, two-ended FP32 solve
+  LK_F64_TILE_F32_TWIST = 12,  // filter: FP64 field, two-ended FP32 solve
+  LK_F64_1L = 13               // FP64 one-lane sweeps with FMA (fast mode)
 };
+// the one-lane sweeps (k_line)
+inline bool kind_one_lane(int kind) {
+  return kind == LK_F64 || kind == LK_F64_1L || kind == LK_F32_1L || kind == LK_F64_TILE_F32_SOLVE_1L;
+}
 inline bool kind_quad(int kind) { return kind == LK_F64_QUAD || kind == LK_F32_QUAD; }
 inline bool kind_twist(int kind) {
   return kind == LK_F64_TWIST || kind == LK_F32_TWIST || kind == LK_F64_TILE_F32_TWIST;
@@ -549,6 +554,39 @@ void chunking_dir(int dir, int L, int& nc, int& cr, int nc_req = 0) {
 }
 
 // ---- line task construction ----------------------------------------------------
+constexpr int kLineSmemMax = 227 * 1024;  // the largest dynamic shared memory a line kernel's CTA may request (sm_100a)
+
+// bytes of a one-lane tile without its staged factors
+size_t one_lane_bytes(int dir, const LineTask& t, size_t es) {
+  return kLineHead + (dir == 0 ? (size_t)kLanes * (t.xt ? t.nbox : 1) * t.pitch * es + kLineSlack
+                               : (size_t)t.nbox * t.by * kLanes * es);
+}
+
+// The tile of a one-lane task (dir, L, c0 and the chunks set): the xi line
+// pitch, whether an xi tile moves as tensor boxes (at most `boxes`, each at most
+// 256 elements wide; longer lines take one bulk copy each), and how many
+// factor rows are staged: up to the block of eight past the first constant
+// row, at most kLineStage rows (a slowly converging filter reads the rest from
+// the tables), and no more than the CTA's shared memory leaves.
+void one_lane_tile(int dir, int kind, LineTask& t, int boxes) {
+  const size_t es = tile_elem(kind), rs = kind == LK_F64 || kind == LK_F64_1L ? sizeof(double) : sizeof(float);
+  auto pitch = [&](int n) { return es == 4 ? dir1_pitch<float>(n) : dir1_pitch<double>(n); };
+  t.pitch = dir != 0 ? 0 : pitch(t.L);
+  t.xt = 0;
+  if (dir == 0) {
+    for (int nb = 1; nb <= boxes && !t.xt; ++nb) {
+      const int w = pitch((t.L + nb - 1) / nb);
+      // both boxes keep the 13 positions the closures read
+      if (w > 256 || t.L - (nb - 1) * w < 13) continue;
+      t.xt = 1;
+      t.nbox = nb;
+      t.by = t.pitch = w;
+    }
+  }
+  const size_t used = one_lane_bytes(dir, t, es), row = 6 * rs;
+  const size_t room = used < (size_t)kLineSmemMax ? ((size_t)kLineSmemMax - used) / row : 0;
+  t.ts = (int)std::min<size_t>(std::min<size_t>(std::min(t.L, kLineStage), (size_t)t.c0 + 12), room);
+}
 // Both ends of direction dir periodic onto the block itself: the interface
 // contraction of a derivative pass can be formed inside the line kernel.
 bool self_periodic(const BlockGeom& g, int dir) {
@@ -567,7 +605,7 @@ void fill_line_task(const canard_ctx* c, const BlockState& B, int dir /*0..2*/, 
   t.in = in;
   t.out = out;
   const bool f64solve = kind == LK_F64 || kind == LK_F64_TM || kind == LK_F64_SPLIT || kind == LK_F64_QUAD ||
-                        kind == LK_F64_TWIST;
+                        kind == LK_F64_TWIST || kind == LK_F64_1L;
   t.lu = (kind == LK_F64_SPLIT || kind == LK_F64_QUAD) ? static_cast<const void*>(B.lu64s[nt][dir])
          : kind == LK_F64_TWIST                        ? static_cast<const void*>(B.lu64t[nt][dir])
          : kind_twist(kind)                            ? static_cast<const void*>(B.lu32t[nt][dir])
@@ -615,6 +653,8 @@ void fill_line_task(const canard_ctx* c, const BlockState& B, int dir /*0..2*/, 
     t.kf = B.kf32[nt][dir];
   }
   chunking_dir(dir, t.L, t.nbox, t.by, nc_req);
+  // an increment along xi goes out by one bulk add per line: one box at most
+  if (kind_one_lane(kind)) one_lane_tile(dir, kind, t, nt == 1 && kind != LK_F64_1L ? 1 : 2);
   if (kind == LK_F64_TM) {  // 32-row boxes streamed through the ring
     t.by = kTmChunk;
     t.nbox = (t.L + kTmChunk - 1) / kTmChunk;
@@ -640,10 +680,6 @@ void fill_line_task(const canard_ctx* c, const BlockState& B, int dir /*0..2*/, 
   }
 }
 
-// the largest dynamic shared memory a line kernel's CTA may request (sm_100a:
-// 227 KiB per block)
-constexpr int kLineSmemMax = 227 * 1024;
-
 // dynamic shared memory of one task's tile
 size_t line_smem(int dir, const LineTask& t, int kind) {
   if (kind == LK_F64_TM) return kTmSmem;
@@ -656,6 +692,9 @@ size_t line_smem(int dir, const LineTask& t, int kind) {
     const int P = kind_f32_fields(kind) ? dir1_pitch<float>(t.L) : dir1_pitch<double>(t.L);
     return 128 + twist_tile_bytes(dir, t.L, t.nbox, t.by, es, P) + (size_t)2 * 5 * kTwistSh * rs;
   }
+  if (kind_one_lane(kind))
+    return one_lane_bytes(dir, t, es) +
+           (kind == LK_F64 || kind == LK_F64_1L ? line_tab_bytes<double>(t.ts) : line_tab_bytes<float>(t.ts));
   if (dir == 0)
     return 128 + (size_t)lanes * (kind_f32_fields(kind) ? dir1_pitch<float>(t.L) : dir1_pitch<double>(t.L)) * es;
   return 128 + (size_t)t.nbox * t.by * lanes * es;
@@ -666,6 +705,7 @@ size_t tile_smem_for(int dir, int L, int kind) {
   LineTask t{};
   t.L = L;
   chunking_dir(dir, L, t.nbox, t.by);
+  if (kind_one_lane(kind)) one_lane_tile(dir, kind, t, 0);
   return line_smem(dir, t, kind);
 }
 
@@ -714,13 +754,14 @@ EncodeTiledFn encode_fn() {
 }
 
 // 3-D map over a padded field (X, Y, Z) with box (32, by, 1) for eta lines or
-// (32, 1, by) for zeta lines.
+// (32, 1, by) for zeta lines; dir 0: box (lanes, by, 1) over the plane of all
+// xi lines (Y of them, Z = 1).
 CUtensorMap field_map(const void* base, int X, int Y, int Z, int Xp, int dir, int by, size_t es = sizeof(double),
                       int lanes = kLanes) {
   CUtensorMap m;
   cuuint64_t dims[3] = {(cuuint64_t)X, (cuuint64_t)Y, (cuuint64_t)Z};
   cuuint64_t strides[2] = {(cuuint64_t)Xp * es, (cuuint64_t)Xp * Y * es};
-  cuuint32_t box[3] = {(cuuint32_t)lanes, (cuuint32_t)(dir == 1 ? by : 1), (cuuint32_t)(dir == 2 ? by : 1)};
+  cuuint32_t box[3] = {(cuuint32_t)lanes, (cuuint32_t)(dir == 2 ? 1 : by), (cuuint32_t)(dir == 2 ? by : 1)};
   cuuint32_t estr[3] = {1, 1, 1};
   const CUtensorMapDataType ty = es == sizeof(float) ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
   CUresult r = encode_fn()(&m, ty, 3, const_cast<void*>(base), dims, strides, box, estr,
@@ -758,7 +799,15 @@ Table<LineTask> make_line_table(canard_ctx* c, std::vector<LineTask> v, int dir,
   T.tasks = dupload(v, c->st);
   T.first = dupload(tile_task, c->st);
   std::vector<CUtensorMap> maps(2 * v.size());
-  if (dir != 0)
+  if (dir == 0 && kind_one_lane(kind)) {
+    std::memset(maps.data(), 0, maps.size() * sizeof(CUtensorMap));
+    for (size_t i = 0; i < v.size(); ++i)
+      if (v[i].xt) {  // all of the block's xi lines as rows of one plane
+        const LineTask& t = v[i];
+        maps[2 * i] = field_map(t.in, t.X, t.Y * t.Z, 1, t.Xp, 0, kLanes, es, t.pitch);
+        maps[2 * i + 1] = field_map(t.out, t.X, t.Y * t.Z, 1, t.Xp, 0, kLanes, es, t.pitch);
+      }
+  } else if (dir != 0)
     for (size_t i = 0; i < v.size(); ++i) {
       maps[2 * i] = field_map(v[i].in, v[i].X, v[i].Y, v[i].Z, v[i].Xp, dir, v[i].by, es, tile_lanes(kind));
       maps[2 * i + 1] = field_map(v[i].out, v[i].X, v[i].Y, v[i].Z, v[i].Xp, dir, v[i].by, es, tile_lanes(kind));
@@ -796,11 +845,11 @@ Table<T> make_lines_table(canard_ctx* c, std::vector<T> v, bool transient, int T
   return Tb;
 }
 
-template <int DIR, int OP, class TT, class RS>
+template <int DIR, int OP, class TT, class RS, int V>
 void launch_line_dir(canard_ctx* c, const Table<LineTask>& T) {
   if (T.ntasks == 0 || T.total == 0) return;
   Timed tm(c, (OP == 0 ? T_DERIV_XI : T_FILTER_XI) + DIR - 1, T.bytes);
-  launch_line_t<DIR, OP, TT, RS>(T.total, T.smem, c->st, T.tasks, T.first, T.tdiv, T.maps, c->derr);
+  launch_line_t<DIR, OP, TT, RS, V>(T.total, T.smem, c->st, T.tasks, T.first, T.tdiv, T.maps, c->derr);
   CK(cudaGetLastError());
 }
 
@@ -858,12 +907,13 @@ void launch_filt2s_dir(canard_ctx* c, const Table<LineTask>& T) {
 
 template <int DIR, int OP>
 void launch_line_kind(canard_ctx* c, const Table<LineTask>& T) {
-  if (T.kind == LK_F64) launch_line_dir<DIR, OP, double, double>(c, T);
+  if (T.kind == LK_F64) launch_line_dir<DIR, OP, double, double, 0>(c, T);
+  else if (T.kind == LK_F64_1L) launch_line_dir<DIR, OP, double, double, 1>(c, T);
   else if (DIR != 1 && T.kind == LK_F64_TM) launch_line_tm_dir<(DIR == 1 ? 2 : DIR), OP>(c, T);
   else if (OP == 0 && T.kind == LK_F32) launch_line2_dir<DIR, 0, float>(c, T);
   else if (OP == 1 && T.kind == LK_F64_TILE_F32_SOLVE) launch_line2_dir<DIR, 1, double>(c, T);
-  else if (OP == 0 && T.kind == LK_F32_1L) launch_line_dir<DIR, 0, float, float>(c, T);
-  else if (OP == 1 && T.kind == LK_F64_TILE_F32_SOLVE_1L) launch_line_dir<DIR, 1, double, float>(c, T);
+  else if (OP == 0 && T.kind == LK_F32_1L) launch_line_dir<DIR, 0, float, float, 1>(c, T);
+  else if (OP == 1 && T.kind == LK_F64_TILE_F32_SOLVE_1L) launch_line_dir<DIR, 1, double, float, 1>(c, T);
   else if (OP == 1 && T.kind == LK_F64_STREAM_F32) launch_filt2s_dir<DIR>(c, T);
   else if (T.kind == LK_F64_SPLIT) launch_line2_dir<DIR, OP, double, double>(c, T);
   else if (OP == 0 && T.kind == LK_F64_QUAD) launch_line4_dir<DIR, double, double>(c, T);
@@ -897,24 +947,30 @@ void set_line_smem_limits() {
   std::lock_guard<std::mutex> lk(mu);
   if (done_dev[dev]) return;
   const int lim = kLineSmemMax;
-  CK((line_smem_limit<1, 0, double, double>(lim)));
-  CK((line_smem_limit<2, 0, double, double>(lim)));
-  CK((line_smem_limit<3, 0, double, double>(lim)));
-  CK((line_smem_limit<1, 1, double, double>(lim)));
-  CK((line_smem_limit<2, 1, double, double>(lim)));
-  CK((line_smem_limit<3, 1, double, double>(lim)));
+  CK((line_smem_limit<1, 0, double, double, 0>(lim)));
+  CK((line_smem_limit<2, 0, double, double, 0>(lim)));
+  CK((line_smem_limit<3, 0, double, double, 0>(lim)));
+  CK((line_smem_limit<1, 1, double, double, 0>(lim)));
+  CK((line_smem_limit<2, 1, double, double, 0>(lim)));
+  CK((line_smem_limit<3, 1, double, double, 0>(lim)));
   CK((line2_smem_limit<1, 0, float>(lim)));
   CK((line2_smem_limit<2, 0, float>(lim)));
   CK((line2_smem_limit<3, 0, float>(lim)));
   CK((line2_smem_limit<1, 1, double>(lim)));
   CK((line2_smem_limit<2, 1, double>(lim)));
   CK((line2_smem_limit<3, 1, double>(lim)));
-  CK((line_smem_limit<1, 0, float, float>(lim)));
-  CK((line_smem_limit<2, 0, float, float>(lim)));
-  CK((line_smem_limit<3, 0, float, float>(lim)));
-  CK((line_smem_limit<1, 1, double, float>(lim)));
-  CK((line_smem_limit<2, 1, double, float>(lim)));
-  CK((line_smem_limit<3, 1, double, float>(lim)));
+  CK((line_smem_limit<1, 0, float, float, 1>(lim)));
+  CK((line_smem_limit<2, 0, float, float, 1>(lim)));
+  CK((line_smem_limit<3, 0, float, float, 1>(lim)));
+  CK((line_smem_limit<1, 1, double, float, 1>(lim)));
+  CK((line_smem_limit<2, 1, double, float, 1>(lim)));
+  CK((line_smem_limit<3, 1, double, float, 1>(lim)));
+  CK((line_smem_limit<1, 0, double, double, 1>(lim)));
+  CK((line_smem_limit<2, 0, double, double, 1>(lim)));
+  CK((line_smem_limit<3, 0, double, double, 1>(lim)));
+  CK((line_smem_limit<1, 1, double, double, 1>(lim)));
+  CK((line_smem_limit<2, 1, double, double, 1>(lim)));
+  CK((line_smem_limit<3, 1, double, double, 1>(lim)));
   CK((line_tm_smem_limit<2, 0>()));
   CK((line_tm_smem_limit<3, 0>()));
   CK((line_tm_smem_limit<2, 1>()));
@@ -1456,14 +1512,34 @@ bool twist_ok(const canard_ctx* c, int dir, int kind) {
   return true;
 }
 
-// Defaults without autotuning: the two-ended solve where the lines admit it
-// (fast mode: the fastest FP64 filter and derivative at 257 points; mixed
-// precision: the fastest filter), else the split solve
+// the longest line of direction dir over the context's blocks
+int longest_line(const canard_ctx* c, int dir) {
+  int L = 0;
+  for (const auto& b : c->blocks) L = std::max(L, b.g.ijk[0][dir] + 1);
+  return L;
+}
+
+// Defaults without autotuning, five fields, ms per launch on a B200. The
+// one-lane sweeps keep whole lines of 32 in a CTA, so their rate falls where
+// fewer than four tiles fit an SM (FP64: lines of more than about 200 points);
+// the two-ended solve halves the dependent chain there at the price of more
+// start-up per tile.
+// Fast mode, derivative, one-lane against two-ended: 65 points (zeta of
+// 193 x 129 x 65) 0.040 / 0.057, 129 points 0.039 / 0.048, 193 points 0.047 /
+// 0.054, 257 points 0.294-0.319 / 0.300-0.306, 385 points 0.295 / 0.274.
+// Fast mode, filter: 65 points 0.038 / 0.054, 129 points 0.040 / 0.049, 193
+// points 0.049 / 0.047, 257 points 0.39-0.49 / 0.34-0.42.
+// Mixed precision, derivative, one-lane against split: 65 points 0.027 /
+// 0.046, 129 points 0.025 / 0.033, 257 points 0.139-0.147 / 0.167-0.189, 385
+// points 0.125 / 0.135. Its filter runs in FP64 like the fast mode's where the
+// two-ended FP32 elimination is the slower one (257 points 0.34-0.43 / 0.36-0.50).
 int default_kind(const canard_ctx* c, int grp, int dir) {
-  if (c->fast()) return twist_ok(c, dir, LK_F64_TWIST) ? LK_F64_TWIST : LK_F64_SPLIT;
-  if (!c->f32()) return LK_F64;
-  if (grp == 0) return twist_ok(c, dir, LK_F64_TILE_F32_TWIST) ? LK_F64_TILE_F32_TWIST : LK_F64_TILE_F32_SOLVE;
-  return LK_F32;
+  if (!c->fast() && !c->f32()) return LK_F64;
+  const int L = longest_line(c, dir);
+  auto fits = [&](int kind) { return tile_smem_for(dir, L, kind) <= (size_t)kLineSmemMax; };
+  if (c->f32() && grp != 0) return fits(LK_F32_1L) ? LK_F32_1L : LK_F32;
+  if (twist_ok(c, dir, LK_F64_TWIST) && L > (grp == 0 ? 160 : 200)) return LK_F64_TWIST;
+  return fits(LK_F64_1L) ? LK_F64_1L : LK_F64_SPLIT;
 }
 
 int group_kind(const canard_ctx* c, int grp, int dir) {
@@ -2782,6 +2858,7 @@ int canard_autotune(canard_ctx* c, int32_t reps, double* report, int32_t nmax) {
         std::vector<int> kinds{default_kind(c, grp, dir)};
         if (c->fast()) {  // the one-lane and split FP64 sweeps compete in the fast mode
           kinds.push_back(LK_F64);
+          kinds.push_back(LK_F64_1L);
           kinds.push_back(LK_F64_SPLIT);
         }
         if (grp != 0 && c->fast() && quad_ok(c, dir, LK_F64_QUAD)) kinds.push_back(LK_F64_QUAD);
@@ -2798,6 +2875,7 @@ int canard_autotune(canard_ctx* c, int32_t reps, double* report, int32_t nmax) {
         // kind; the FP64 eliminations (one-lane and split) compete with the FP32 ones there
         if (c->f32() && grp == 0) {
           kinds.push_back(LK_F64);
+          kinds.push_back(LK_F64_1L);
           kinds.push_back(LK_F64_SPLIT);
           if (twist_ok(c, dir, LK_F64_TWIST)) kinds.push_back(LK_F64_TWIST);
         }
@@ -2842,17 +2920,17 @@ int canard_autotune(canard_ctx* c, int32_t reps, double* report, int32_t nmax) {
 
 int canard_set_line_kind(canard_ctx* c, int32_t group, int32_t dir, int32_t kind, int32_t chunks) {
   return guarded(c, [&] {
-    if (group < 0 || group > 2 || dir < 0 || dir > 2 || kind < -1 || kind > LK_F64_TILE_F32_TWIST || chunks < 0 ||
+    if (group < 0 || group > 2 || dir < 0 || dir > 2 || kind < -1 || kind > LK_F64_1L || chunks < 0 ||
         chunks == 1 || chunks > kMaxChunks || (dir == 0 && chunks != 0))
       throw ApiError(CANARD_ERR_ARG, "bad line kind argument");
     if (kind >= 0) {
       bool fits;
       if (!c->f32())
-        fits = kind == LK_F64 || kind == LK_F64_SPLIT || (kind == LK_F64_TM && tm_ok(c, dir) && chunks == 0) ||
+        fits = kind == LK_F64 || kind == LK_F64_1L || kind == LK_F64_SPLIT || (kind == LK_F64_TM && tm_ok(c, dir) && chunks == 0) ||
                (kind == LK_F64_QUAD && group != 0 && quad_ok(c, dir, kind)) ||
                (kind == LK_F64_TWIST && twist_ok(c, dir, kind));
       else if (group == 0)
-        fits = kind == LK_F64_TILE_F32_SOLVE || kind == LK_F64_TILE_F32_SOLVE_1L || kind == LK_F64 ||
+        fits = kind == LK_F64_TILE_F32_SOLVE || kind == LK_F64_TILE_F32_SOLVE_1L || kind == LK_F64 || kind == LK_F64_1L ||
                kind == LK_F64_SPLIT || (kind == LK_F64_STREAM_F32 && chunks == 0) ||
                ((kind == LK_F64_TWIST || kind == LK_F64_TILE_F32_TWIST) && twist_ok(c, dir, kind));
       else
@@ -3057,6 +3135,7 @@ extern "C" int canard_deriv_noalloc(const double* d_in, double* d_out, int32_t l
     t.X = g.X; t.Y = g.Y; t.Z = g.Z; t.Xp = g.Xp;
     t.L = L; t.nbs = nbs; t.m = 1; t.ndf0 = n0; t.ndf1 = n1;
     chunking_dir(dir, L, t.nbox, t.by);
+    one_lane_tile(dir, LK_F64, t, 0);
     if (dir == 0) {
       t.ntx = 1;
       t.ntiles = (g.Y * g.Z + kLanes - 1) / kLanes;
@@ -3120,9 +3199,9 @@ extern "C" int canard_deriv_noalloc(const double* d_in, double* d_out, int32_t l
     const CUtensorMap* dm = reinterpret_cast<const CUtensorMap*>(base + kNaMaps);
     int* de = reinterpret_cast<int*>(base + kNaErr);
     // one task: every tile's task is tile / ntiles = 0 (the zero table is not read)
-    if (dir == 0) launch_line_t<1, 0, double, double>(t.ntiles, smem, st, dt, d0, t.ntiles, dm, de);
-    else if (dir == 1) launch_line_t<2, 0, double, double>(t.ntiles, smem, st, dt, d0, t.ntiles, dm, de);
-    else launch_line_t<3, 0, double, double>(t.ntiles, smem, st, dt, d0, t.ntiles, dm, de);
+    if (dir == 0) launch_line_t<1, 0, double, double, 0>(t.ntiles, smem, st, dt, d0, t.ntiles, dm, de);
+    else if (dir == 1) launch_line_t<2, 0, double, double, 0>(t.ntiles, smem, st, dt, d0, t.ntiles, dm, de);
+    else launch_line_t<3, 0, double, double, 0>(t.ntiles, smem, st, dt, d0, t.ntiles, dm, de);
     CK(cudaGetLastError());
   } catch (const ApiError& e) {
     return fail(e.code, e.what());

@@ -102,6 +102,9 @@ struct LineTask {
   int q2, q3;              // quad split: first rows of the third and fourth segments (h: of the second)
   int tile0, ntiles, ntx;  // first global tile, tiles, x-tiles per row (dir 2/3)
   int nbox, by;            // chunks per tile and positions per chunk
+  // one-lane sweeps: staged factor rows; xi tiles: line pitch, and whether a
+  // tile moves as one tensor box
+  int ts, pitch, xt;
 };
 
 // Interface contraction of one face (t_numerics%mpigo): the sender's face
@@ -258,21 +261,7 @@ __device__ __forceinline__ double pow15(double x) {
 // The LU factors of the Toeplitz interior converge to a fixed point: rows
 // [c0, L-4] hold bitwise identical factors (found on the host), which the
 // sweeps keep in registers. Only the closure rows near the ends read the
-// factor tables, so the dependent chain carries no memory latency there.
-template <class RS>
-struct LuRows {
-  const RS* __restrict__ l1;
-  const RS* __restrict__ l2;
-  const RS* __restrict__ u1;
-  const RS* __restrict__ u2;
-  const RS* __restrict__ u3;
-  RS cl1, cl2, cu1, cu2, cu3;
-  int c0, c1;
-  __device__ __forceinline__ LuRows(const RS* lu, int L, RS a, RS b, RS c, RS d, RS e, int c0_)
-      : l1(lu), l2(lu + L), u1(lu + 2 * L), u2(lu + 3 * L), u3(lu + 4 * L), cl1(a), cl2(b), cu1(c), cu2(d),
-        cu3(e), c0(c0_), c1(L - 4) {}
-};
-
+// factor tables.
 constexpr int kMaxChunks = 8;
 
 // While a tile's copies are in flight: the scheme's coefficients (1.2 KB)
@@ -295,23 +284,6 @@ __device__ long long* g_trace;  // per CTA: start, loads issued, data ready, for
 #else
 #define TRACE(k)
 #endif
-
-// A tile arrives in NC chunks of CR positions (rows), chunk 0 and the last
-// chunk first (the closures read both ends), then 1, 2, ...; the forward
-// sweep waits for a chunk only when its look-ahead reaches it.
-struct ChunkIn {
-  uint64_t* bars;
-  int CR, NC, L;
-  int next;   // next middle chunk to wait for
-  int ready;  // rows [0, ready) and the last chunk have arrived
-  __device__ __forceinline__ bool wait_next(int* err) {
-    if (next >= NC - 1) { ready = L; return true; }
-    if (!mbar_wait(bars + next, 0)) { atomicExch(err, kErrTimeout); return false; }
-    ++next;
-    ready = (next >= NC - 1) ? L : next * CR;
-    return true;
-  }
-};
 
 // Factor providers: the interior constants or the per-row tables.
 template <class RS>
@@ -505,308 +477,6 @@ __device__ __forceinline__ void bwd8(TT* __restrict__ s, int i, const CF& cf, RS
   bwd8_c<ST, TT, RS, 0>(s, i, b, o, cp1, cp2);
 }
 
-// A run of forward blocks of eight while COND(i) holds, software-pipelined:
-// one straight-line body forms the next block's right-hand sides (RHS8) and
-// loads its factors while the current block's dependent chain runs, so the
-// scheduler can fill the chain's latency. RHS8(i + 8) reads rows i+8.. that
-// the chain of rows i..i+7 does not write. CONST: register constants, no loads.
-#define FWD_RUN(COND, CF, CONST, RHS8)                                        \
-  if (COND(i)) {                                                              \
-    F8<RS> nx;                                                                \
-    nx.load(CF, i);                                                           \
-    TT rr[8];                                                                 \
-    RHS8(i, rr);                                                              \
-    while (COND(i + 8)) {                                                     \
-      const F8<RS> cu = nx;                                                   \
-      TT rc[8];                                                               \
-      _Pragma("unroll") for (int k = 0; k < 8; ++k) rc[k] = rr[k];            \
-      if (!(CONST)) nx.load(CF, i + 8);                                       \
-      RHS8(i + 8, rr);                                                        \
-      chain8_fwd<ST, TT, RS>(s, i, cu, rc, am2, am1);                         \
-      i += 8;                                                                 \
-    }                                                                         \
-    chain8_fwd<ST, TT, RS>(s, i, nx, rr, am2, am1);                           \
-    i += 8;                                                                   \
-  }
-
-// The same for back substitution blocks: the next block's u1 * (forward
-// result) products, factors and (ADD) originals are formed during the current
-// block's chain; they read rows below the ones the chain writes.
-#define BWD_RUN(COND, CF, CONST)                                              \
-  if (COND(i)) {                                                              \
-    B8<RS> bn;                                                                \
-    O8<TT> on;                                                                \
-    RS pn[8];                                                                 \
-    bn.load(CF, i);                                                           \
-    if (ADD) on.load(og, ogs, i);                                             \
-    bwd_p8<ST, TT, RS>(s, i, bn, pn);                                         \
-    while (COND(i - 8)) {                                                     \
-      const B8<RS> bu = bn;                                                   \
-      const O8<TT> ou = on;                                                   \
-      RS pu[8];                                                               \
-      _Pragma("unroll") for (int k = 0; k < 8; ++k) pu[k] = pn[k];            \
-      if (!(CONST)) bn.load(CF, i - 8);                                       \
-      if (ADD) on.load(og, ogs, i - 8);                                       \
-      bwd_p8<ST, TT, RS>(s, i - 8, bn, pn);                                   \
-      bwd_chain8<ST, TT, RS, ADD>(s, i, bu, pu, ou, cp1, cp2);                \
-      i -= 8;                                                                 \
-    }                                                                         \
-    bwd_chain8<ST, TT, RS, ADD>(s, i, bn, pn, on, cp1, cp2);                  \
-    i -= 8;                                                                   \
-  }
-
-// Drives the forward rows [FIRST, LAST] with look-ahead LA: blocks of eight
-// where the look-ahead rows have arrived, single rows otherwise.
-#define FORWARD_ROWS(FIRST, LAST, LA, RHS8, STEP)                             \
-  {                                                                           \
-    const CoefConst<RS> CC{F.cl1, F.cl2, F.cu1, F.cu2, F.cu3};                \
-    const CoefTable<RS> CT{F.l1, F.l2, F.u1, F.u2, F.u3};                     \
-    int i = (FIRST);                                                          \
-    while (i <= (LAST)) {                                                     \
-      const int e = min((LAST), CI.ready - 1 - (LA));                         \
-      if (e < i) {                                                            \
-        if (!CI.wait_next(err)) return false;                                 \
-        __syncwarp();                                                         \
-        continue;                                                             \
-      }                                                                       \
-      {                                                                       \
-        const int h = min(F.c0, e + 1);                                       \
-        FWD_RUN(FR_H, CT, false, RHS8)                                        \
-        for (; i < h; ++i) STEP(CT.L1(i), CT.L2(i))                           \
-        const int ce = min(F.c1, e);                                          \
-        FWD_RUN(FR_CE, CC, true, RHS8)                                        \
-        FWD_RUN(FR_E, CT, false, RHS8)                                        \
-        for (; i <= e; ++i) STEP(CT.L1(i), CT.L2(i))                          \
-      }                                                                       \
-    }                                                                         \
-  }
-
-#define FR_H(x) ((x) + 7 < h)
-#define FR_CE(x) ((x) + 7 <= ce)
-#define FR_E(x) ((x) + 7 <= e)
-#define BR_TOP(x) ((x) > F.c1 && (x) - 7 >= lo)
-#define BR_CE(x) ((x) - 7 >= ce)
-#define BR_LO(x) ((x) - 7 >= lo)
-
-// Back substitution over rows N-2 .. 0; after the lowest row of chunk c the
-// chunk is final and DONE(c) runs (stores it). With ADD (filter) every row is
-// stored as original + increment (OUT).
-#define OUT(i, v) (ADD ? __ldg(og + (long long)(i) * ogs) + TT(v) : TT(v))
-#define BACKWARD_ROWS(DONE)                                                   \
-  {                                                                           \
-    const CoefConst<RS> CC{F.cl1, F.cl2, F.cu1, F.cu2, F.cu3};                \
-    const CoefTable<RS> CT{F.l1, F.l2, F.u1, F.u2, F.u3};                     \
-    RS cp1 = CT.U1(N) * RS(S(N));                                             \
-    S(N) = OUT(N, cp1);                                                       \
-    RS c = CT.U1(N - 1) * RS(S(N - 1)) - CT.U2(N - 1) * cp1;                  \
-    S(N - 1) = OUT(N - 1, c);                                                 \
-    RS cp2 = cp1;                                                             \
-    cp1 = c;                                                                  \
-    int i = N - 2;                                                            \
-    for (int ch = CI.NC - 1; ch >= 0; --ch) {                                 \
-      const int lo = ch * CI.CR;                                              \
-      BWD_RUN(BR_TOP, CT, false)                                              \
-      {                                                                       \
-        const int ce = max(F.c0, lo);                                         \
-        BWD_RUN(BR_CE, CC, true)                                              \
-      }                                                                       \
-      BWD_RUN(BR_LO, CT, false)                                               \
-      for (; i >= lo; --i) {                                                  \
-        c = (CT.U1(i) * RS(S(i)) - CT.U2(i) * cp1) - CT.U3(i) * cp2;          \
-        S(i) = OUT(i, c);                                                     \
-        cp2 = cp1;                                                            \
-        cp1 = c;                                                              \
-      }                                                                       \
-      DONE(ch);                                                               \
-    }                                                                         \
-  }
-
-// Compact first derivative of one line held in shared memory with element
-// stride ST (src/mo_numerics.f90:742-792). On return the line holds the
-// derivative; Done(ch) is called as chunks become final. Returns false if a
-// bounded wait gave up.
-template <int ST, class TT, class RS, class Done>
-__device__ __forceinline__ bool sweep_deriv(TT* __restrict__ s, int L, const LuRows<RS>& F, int ndf0, int ndf1,
-                                            const DevScheme* __restrict__ sc, TT r00, TT r10, TT r01, TT r11,
-                                            ChunkIn& CI, int* err, Done&& done) {
-#define S(i) s[(i)*ST]
-  constexpr int ADD = 0;
-  const TT* og = nullptr;
-  const int ogs = 0;
-  const int N = L - 1;
-  TT b0, b1, bn1, bn;
-  if (ndf0 == 0) {
-    const TT s0 = S(0), s1 = S(1), s2 = S(2), s3 = S(3), s4 = S(4);
-    b0 = ((TT(CA_A01) * (s1 - s0) + TT(CA_A02) * (s2 - s0)) + TT(CA_A03) * (s3 - s0)) + TT(CA_A04) * (s4 - s0);
-    b1 = ((TT(CA_A10) * (s0 - s1) + TT(CA_A12) * (s2 - s1)) + TT(CA_A13) * (s3 - s1)) + TT(CA_A14) * (s4 - s1);
-  } else {
-    TT t0 = 0, t1 = 0;
-#pragma unroll
-    for (int i = 0; i < 12; ++i) {
-      const TT v = S(i);
-      t0 = t0 + TT(sc->pbci[0][0][i]) * v;
-      t1 = t1 + TT(sc->pbci[0][1][i]) * v;
-    }
-    b0 = t0 + r00;
-    b1 = t1 + r10;
-  }
-  if (ndf1 == 0) {
-    const TT e0 = S(N), e1 = S(N - 1), e2 = S(N - 2), e3 = S(N - 3), e4 = S(N - 4);
-    bn = ((TT(CA_A01) * (e0 - e1) + TT(CA_A02) * (e0 - e2)) + TT(CA_A03) * (e0 - e3)) + TT(CA_A04) * (e0 - e4);
-    bn1 = ((TT(CA_A10) * (e1 - e0) + TT(CA_A12) * (e1 - e2)) + TT(CA_A13) * (e1 - e3)) + TT(CA_A14) * (e1 - e4);
-  } else {
-    TT t0 = 0, t1 = 0;
-#pragma unroll
-    for (int i = 0; i < 12; ++i) {
-      const TT v = S(N - i);
-      t0 = t0 + TT(sc->pbci[0][0][i]) * v;
-      t1 = t1 + TT(sc->pbci[0][1][i]) * v;
-    }
-    bn = -t0 - r01;
-    bn1 = -t1 - r11;
-  }
-  // forward elimination, in place; originals kept in a register window
-  TT w0 = S(0), w1 = S(1), w2 = S(2), w3 = S(3);
-  RS am2 = RS(b0);
-  RS am1 = RS(b1) - __ldg(F.l2 + 1) * am2;
-  S(0) = TT(am2);
-  S(1) = TT(am1);
-#define FWD(L1, L2)                                                 \
-  {                                                                 \
-    const TT w4 = S(i + 2);                                         \
-    const TT rhs = TT(CA_AA) * (w3 - w1) + TT(CA_AB) * (w4 - w0);   \
-    const RS a = (RS(rhs) - (L1) * am2) - (L2) * am1;               \
-    S(i) = TT(a);                                                   \
-    w0 = w1; w1 = w2; w2 = w3; w3 = w4;                             \
-    am2 = am1; am1 = a;                                             \
-  }
-#define RHS8(I, R) rhs8_deriv<ST, TT>(s, I, w0, w1, w2, w3, R)
-  FORWARD_ROWS(2, N - 2, 2, RHS8, FWD)
-#undef RHS8
-#undef FWD
-  {
-    const RS a = (RS(bn1) - __ldg(F.l1 + N - 1) * am2) - __ldg(F.l2 + N - 1) * am1;
-    S(N - 1) = TT(a);
-    am2 = am1; am1 = a;
-    const RS an = (RS(bn) - __ldg(F.l1 + N) * am2) - __ldg(F.l2 + N) * am1;
-    S(N) = TT(an);
-  }
-  TRACE(3)
-  BACKWARD_ROWS(done)
-#undef S
-  return true;
-}
-
-// Compact filter of one line (src/mo_numerics.f90:922-977): the increment is
-// solved for and each row stored as original + increment, the original read
-// from og[row * ogs] (this lane's line in the unfiltered field).
-// ADD 1: every row is stored as original (og, stride ogs) + increment; ADD 0:
-// the tile receives the increment alone (the caller adds it to the field).
-template <int ST, class TT, class RS, int ADD, class Done>
-__device__ __forceinline__ bool sweep_filter(TT* __restrict__ s, int L, const LuRows<RS>& F, int ndf0, int ndf1,
-                                             const DevScheme* __restrict__ sc, TT r00, TT r10, TT r20, TT r01,
-                                             TT r11, TT r21, const TT* __restrict__ og, int ogs,
-                                             ChunkIn& CI, int* err, Done&& done) {
-#define S(i) s[(i)*ST]
-  const int N = L - 1;
-  const TT fa = TT(sc->fa), fb = TT(sc->fb), fc = TT(sc->fc);
-  auto fbc = [&](int r, int k) { return TT(sc->fbc[r][k]); };
-  TT b0, b1, b2, bn2, bn1, bn;
-  if (ndf0 == 0) {
-    const TT s0 = S(0), s1 = S(1), s2 = S(2), s3 = S(3), s4 = S(4), s5 = S(5);
-    b0 = (((fbc(0, 0) * (s1 - s0) + fbc(0, 1) * (s2 - s0)) + fbc(0, 2) * (s3 - s0)) + fbc(0, 3) * (s4 - s0)) +
-         fbc(0, 4) * (s5 - s0);
-    b1 = (((fbc(1, 0) * (s0 - s1) + fbc(1, 1) * (s2 - s1)) + fbc(1, 2) * (s3 - s1)) + fbc(1, 3) * (s4 - s1)) +
-         fbc(1, 4) * (s5 - s1);
-    b2 = (((fbc(2, 0) * (s0 - s2) + fbc(2, 1) * (s1 - s2)) + fbc(2, 2) * (s3 - s2)) + fbc(2, 3) * (s4 - s2)) +
-         fbc(2, 4) * (s5 - s2);
-  } else {
-    TT t0 = 0, t1 = 0;
-#pragma unroll
-    for (int i = 0; i < 12; ++i) {
-      const TT v = S(i);
-      t0 = t0 + TT(sc->pbci[1][0][i]) * v;
-      t1 = t1 + TT(sc->pbci[1][1][i]) * v;
-    }
-    const TT s0 = S(0), s1 = S(1), s2 = S(2), s3 = S(3), s4 = S(4), s5 = S(5);
-    const TT ra2 = s2 + s2;
-    b0 = t0 + r00;
-    b1 = t1 + r10;
-    b2 = (fa * ((s1 + s3) - ra2) + fb * ((s0 + s4) - ra2)) + fc * ((r20 + s5) - ra2);
-  }
-  if (ndf1 == 0) {
-    const TT e0 = S(N), e1 = S(N - 1), e2 = S(N - 2), e3 = S(N - 3), e4 = S(N - 4), e5 = S(N - 5);
-    bn = (((fbc(0, 0) * (e1 - e0) + fbc(0, 1) * (e2 - e0)) + fbc(0, 2) * (e3 - e0)) + fbc(0, 3) * (e4 - e0)) +
-         fbc(0, 4) * (e5 - e0);
-    bn1 = (((fbc(1, 0) * (e0 - e1) + fbc(1, 1) * (e2 - e1)) + fbc(1, 2) * (e3 - e1)) + fbc(1, 3) * (e4 - e1)) +
-          fbc(1, 4) * (e5 - e1);
-    bn2 = (((fbc(2, 0) * (e0 - e2) + fbc(2, 1) * (e1 - e2)) + fbc(2, 2) * (e3 - e2)) + fbc(2, 3) * (e4 - e2)) +
-          fbc(2, 4) * (e5 - e2);
-  } else {
-    TT t0 = 0, t1 = 0;
-#pragma unroll
-    for (int i = 0; i < 12; ++i) {
-      const TT v = S(N - i);
-      t0 = t0 + TT(sc->pbci[1][0][i]) * v;
-      t1 = t1 + TT(sc->pbci[1][1][i]) * v;
-    }
-    const TT e0 = S(N), e1 = S(N - 1), e2 = S(N - 2), e3 = S(N - 3), e4 = S(N - 4), e5 = S(N - 5);
-    const TT ra2 = e2 + e2;
-    bn = t0 + r01;
-    bn1 = t1 + r11;
-    bn2 = (fa * ((e3 + e1) - ra2) + fb * ((e4 + e0) - ra2)) + fc * ((e5 + r21) - ra2);
-  }
-  // forward elimination: rows 0..2 from the closures, 3..N-3 interior
-  TT w0 = S(0), w1 = S(1), w2 = S(2), w3 = S(3), w4 = S(4), w5 = S(5);  // s[i-3..i+2] at i = 3
-  RS am2 = RS(b0);
-  RS am1 = RS(b1) - __ldg(F.l2 + 1) * am2;
-  const RS a2 = (RS(b2) - __ldg(F.l1 + 2) * am2) - __ldg(F.l2 + 2) * am1;
-  S(0) = TT(am2);
-  S(1) = TT(am1);
-  S(2) = TT(a2);
-  am2 = am1;
-  am1 = a2;
-#define FWD(L1, L2)                                                                                       \
-  {                                                                                                       \
-    const TT w6 = S(i + 3);                                                                               \
-    const TT rk = w3 + w3;                                                                                \
-    const TT rhs = (fa * ((w2 + w4) - rk) + fb * ((w1 + w5) - rk)) + fc * ((w0 + w6) - rk);               \
-    const RS a = (RS(rhs) - (L1) * am2) - (L2) * am1;                                                     \
-    S(i) = TT(a);                                                                                         \
-    w0 = w1; w1 = w2; w2 = w3; w3 = w4; w4 = w5; w5 = w6;                                                 \
-    am2 = am1; am1 = a;                                                                                   \
-  }
-#define RHS8(I, R) rhs8_filter<ST, TT>(s, I, fa, fb, fc, w0, w1, w2, w3, w4, w5, R)
-  FORWARD_ROWS(3, N - 3, 3, RHS8, FWD)
-#undef RHS8
-#undef FWD
-  {
-    RS a = (RS(bn2) - __ldg(F.l1 + N - 2) * am2) - __ldg(F.l2 + N - 2) * am1;
-    S(N - 2) = TT(a);
-    am2 = am1; am1 = a;
-    a = (RS(bn1) - __ldg(F.l1 + N - 1) * am2) - __ldg(F.l2 + N - 1) * am1;
-    S(N - 1) = TT(a);
-    am2 = am1; am1 = a;
-    a = (RS(bn) - __ldg(F.l1 + N) * am2) - __ldg(F.l2 + N) * am1;
-    S(N) = TT(a);
-  }
-  TRACE(3)
-  BACKWARD_ROWS(done)
-#undef S
-  return true;
-}
-#undef FORWARD_ROWS
-#undef BACKWARD_ROWS
-#undef OUT
-#undef FWD_RUN
-#undef BWD_RUN
-#undef FR_H
-#undef FR_CE
-#undef FR_E
-#undef BR_TOP
-#undef BR_CE
-#undef BR_LO
-
 // The task of this CTA's tile: tdiv > 0 when every task of the launch has
 // tdiv tiles (no table read on the CTA's start-up path), else the table.
 __device__ __forceinline__ int tile_of(const int* __restrict__ tile_task, int tdiv) {
@@ -839,187 +509,7 @@ __host__ __device__ __forceinline__ int dir1_pitch(int L) {
   return p;
 }
 
-// One CTA = one warp = 32 lines. DIR: 1 xi, 2 eta, 3 zeta. OP: 0 derivative,
-// 1 filter (in place, f += increment). TT: field and tile type, RS: type of
-// the elimination. The tile moves in chunks (see ChunkIn): loads overlap the
-// forward sweep, stores the back substitution.
-template <int DIR, int OP, class TT, class RS>
-__global__ void __maxnreg__(200) k_line(const LineTask* __restrict__ tasks, const int* __restrict__ tile_task,
-                                             int tdiv, const CUtensorMap* __restrict__ maps,
-                                             int* __restrict__ err) {
-  constexpr int kVec = 16 / (int)sizeof(TT);  // elements per 16 bytes
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw);
-  TT* s = reinterpret_cast<TT*>(smem_raw + 128);
-  const int lane = threadIdx.x;
-  TRACE(0)
-  // the tile's task and the error flag load together (independent)
-  const int ti = tile_of(tile_task, tdiv);
-  const int eflag = error_flag_early(err);
-  const LineTask& T = tasks[ti];
-  const TT* in = static_cast<const TT*>(T.in);
-  TT* out = static_cast<TT*>(T.out);
-  const int lt = blockIdx.x - T.tile0;
-  const int L = T.L;
-  const int X = T.X, Y = T.Y, Z = T.Z, Xp = T.Xp;
-  const int NC = T.nbox, CR = T.by;
-  int nval, x0 = 0, r0 = 0, fix = 0;  // fix: z for dir 2, y for dir 3
-  if (DIR == 1) {
-    r0 = lt * kLanes;
-    nval = min(kLanes, Y * Z - r0);
-  } else {
-    fix = lt / T.ntx;
-    x0 = (lt % T.ntx) * kLanes;
-    nval = min(kLanes, X - x0);
-  }
-  const int P = dir1_pitch<TT>(L);
-  const long long pstride = (DIR == 2) ? (long long)Xp : (long long)Xp * Y;  // dir 2/3 position stride
-  const long long base = (DIR == 1) ? (long long)r0 * Xp
-                                    : ((DIR == 2) ? (long long)fix * Y * Xp + x0 : (long long)fix * Xp + x0);
-  const CUtensorMap* map_in = maps + 2 * ti;
-  const CUtensorMap* map_out = maps + 2 * ti + 1;
-  auto chunk_len = [&](int c) { return min(CR, L - c * CR); };
-  if (lane == 0) {
-    for (int c = 0; c < NC; ++c) mbar_init(bars + c, 1);
-    mbar_init_done();
-  }
-  // a kernel launched after a bounded wait gave up does no work
-  if (__shfl_sync(0xffffffffu, eflag, 0) != 0) return;
-  __syncwarp();
-  // issue the loads: chunk 0, the last chunk, then the middle ones
-  for (int k = 0; k < NC; ++k) {
-    const int c = (k == 0) ? 0 : (k == 1 ? NC - 1 : k - 1);
-    if (DIR == 1) {
-      const uint32_t bytes = (uint32_t)((chunk_len(c) + kVec - 1) / kVec * kVec * sizeof(TT));
-      if (lane == 0) mbar_expect_tx(bars + c, bytes * nval);
-      __syncwarp();
-      if (lane < nval)
-        bulk_g2s(s + lane * P + c * CR, in + base + (long long)lane * Xp + c * CR, bytes, bars + c);
-    } else if (lane == 0) {
-      mbar_expect_tx(bars + c, (uint32_t)(CR * kLanes * sizeof(TT)));
-      if (DIR == 2) tma_load_3d(s + c * CR * kLanes, map_in, x0, c * CR, fix, bars + c);
-      else tma_load_3d(s + c * CR * kLanes, map_in, x0, fix, c * CR, bars + c);
-    }
-  }
-  prefetch_sweep_start(T.sc, static_cast<const RS*>(T.lu), L, lane);
-  TRACE(1)
-  // the received interface sums load while the tile's copies are in flight
-  // (the periodic contraction below reads the tile instead)
-  const bool has = lane < nval;
-  int jk = 0;
-  if (DIR == 1) jk = r0 + lane;
-  else if (DIR == 2) jk = (x0 + lane) * Z + fix;
-  else jk = fix * X + x0 + lane;
-  const int nbs = T.nbs;
-  const TT* recv = static_cast<const TT*>(T.recv);
-  TT r00 = 0, r10 = 0, r20 = 0, r01 = 0, r11 = 0, r21 = 0;
-  if (OP == 0 && !T.selfp) {
-    if (has && T.ndf0) { r00 = recv[jk]; r10 = recv[nbs + jk]; }
-    if (has && T.ndf1) { r01 = recv[2 * nbs + jk]; r11 = recv[3 * nbs + jk]; }
-  }
-  if (OP == 1) {
-    if (has && T.ndf0) { r00 = recv[jk]; r10 = recv[nbs + jk]; r20 = recv[2 * nbs + jk]; }
-    if (has && T.ndf1) { r01 = recv[3 * nbs + jk]; r11 = recv[4 * nbs + jk]; r21 = recv[5 * nbs + jk]; }
-  }
-  if (!mbar_wait(bars, 0) || !mbar_wait(bars + NC - 1, 0)) {
-    if (lane == 0) atomicExch(err, kErrTimeout);
-    // copies may still be landing: wait for the other chunks (bounded) before exit
-    for (int c = 1; c < NC - 1; ++c) mbar_wait(bars + c, 0);
-    return;
-  }
-  __syncwarp();
-  TRACE(2)
-  ChunkIn CI{bars, CR, NC, L, 1, (NC > 1 ? CR : L)};
-  if (NC <= 2) CI.ready = L;
-#ifdef CANARD_TRACE_WAITALL
-  while (CI.ready < L) CI.wait_next(err);
-  TRACE(7)
-#endif
-  // The xi filter of FP64 fields (in place) leaves the increment in the tile
-  // and adds it to the field with one bulk FP64 reduce-add per line chunk; the
-  // eta/zeta filters add the originals row by row (a reduce-add per 256-byte
-  // row costs more than the re-read, measured).
-  constexpr bool kRedAdd = OP == 1 && sizeof(TT) == 8 && DIR == 1;
-  if (kRedAdd && (L & 1)) s[lane * P + L] = TT(0);  // the 16-byte tail's pad element adds 0
-  // chunk c is final: store it
-  auto done = [&](int c) {
-    const int lo = c * CR, len = chunk_len(c);
-    fence_proxy_async();
-    __syncwarp();
-    if (kRedAdd) {
-      if (lane < nval) {
-        bulk_s2g_add_f64(out + base + (long long)lane * Xp + lo, s + lane * P + lo,
-                         (uint32_t)((len + kVec - 1) / kVec * kVec * sizeof(TT)));
-        bulk_commit();
-      }
-    } else if (DIR == 1) {
-      if (lane < nval) {
-        bulk_s2g(out + base + (long long)lane * Xp + lo, s + lane * P + lo,
-                 (uint32_t)((len + kVec - 1) / kVec * kVec * sizeof(TT)));
-        bulk_commit();
-      }
-    } else if (lane == 0) {
-      // positions past the block edge (and x past X) are not written
-      if (DIR == 2) tma_store_3d(map_out, x0, lo, fix, s + lo * kLanes);
-      else tma_store_3d(map_out, x0, fix, lo, s + lo * kLanes);
-      bulk_commit();
-    }
-  };
-  bool ok = true;
-  // every lane runs the sweep (lanes past the tile edge on zero-filled or
-  // stale columns) so the chunk hand-offs stay warp-uniform; only lanes with a
-  // line read the receive buffers or write drva
-  constexpr int ST = (DIR == 1) ? 1 : kLanes;
-  TT* sl = (DIR == 1) ? s + lane * P : s + lane;
-  const LuRows<RS> F(static_cast<const RS*>(T.lu), L, RS(T.cl1), RS(T.cl2), RS(T.cu1), RS(T.cu2), RS(T.cu3), T.c0);
-  if (OP == 0) {
-    if (T.selfp) {
-      // The line is periodic onto itself, so the interface contraction the
-      // other end would send (src/mo_numerics.f90:503-518 with n45 = 0) is
-      // formed here from the tile: side 0 receives the sums over positions
-      // N-1..N-12, side 1 over positions 1..12, accumulated in the same order.
-      const DevScheme* sc = T.sc;
-      const int N = L - 1;
-#pragma unroll
-      for (int i = 0; i < 12; ++i) {
-        const TT v = sl[(N - 1 - i) * ST], w = sl[(1 + i) * ST];
-        r00 = r00 + TT(sc->pbco[0][0][i]) * v;
-        r10 = r10 + TT(sc->pbco[0][1][i]) * v;
-        r01 = r01 + TT(sc->pbco[0][0][i]) * w;
-        r11 = r11 + TT(sc->pbco[0][1][i]) * w;
-      }
-    }
-    ok = sweep_deriv<ST, TT, RS>(sl, L, F, T.ndf0, T.ndf1, T.sc, r00, r10, r01, r11, CI, err, done);
-    if (ok && has && T.drva) {
-      TT* drva = static_cast<TT*>(T.drva);
-      drva[jk + (long long)nbs * (T.m - 1)] = sl[0];
-      drva[jk + (long long)nbs * ((T.m - 1) + 5)] = sl[(L - 1) * ST];
-    }
-  } else {
-    // this lane's line of the unfiltered field (lanes without a line read
-    // lane 0's, whose results are not stored)
-    const TT* og = (DIR == 1) ? in + base + (long long)(has ? lane : 0) * Xp : in + base + (has ? lane : 0);
-    const int ogs = (DIR == 1) ? 1 : (int)pstride;
-    ok = sweep_filter<ST, TT, RS, kRedAdd ? 0 : 1>(sl, L, F, T.ndf0, T.ndf1, T.sc, r00, r10, r20, r01, r11, r21,
-                                                   og, ogs, CI, err, done);
-  }
-  // every issued bulk store has to finish reading shared memory before exit;
-  // after a timeout, wait for the chunks still in flight (bounded) instead
-  if (!ok) {
-    for (int c = CI.next; c < NC - 1; ++c) mbar_wait(bars + c, 0);
-    return;
-  }
-  TRACE(4)
-  bulk_wait_read0();
-  TRACE(5)
-#ifdef CANARD_TRACE
-  if (threadIdx.x == 0) {
-    unsigned smid;
-    asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
-    g_trace[(long long)blockIdx.x * 8 + 6] = smid;
-  }
-#endif
-}
+#include "kernels_line.cuh"
 
 // ---------------------------------------------------------------------------
 // Split line solves of the FP32 path. One warp holds 16 lines; lane l owns
@@ -3377,10 +2867,10 @@ template <class T>
 void launch_mpigo_t(int grid, cudaStream_t st, const FaceTask* t, const int* f, int nt, int total) {
   k_mpigo<T><<<grid, 128, 0, st>>>(t, f, nt, total);
 }
-template <int DIR, int OP, class TT, class RS>
+template <int DIR, int OP, class TT, class RS, int V>
 void launch_line_t(int grid, size_t smem, cudaStream_t st, const LineTask* t, const int* f, int nt,
                    const CUtensorMap* maps, int* err) {
-  k_line<DIR, OP, TT, RS><<<grid, kLanes, smem, st>>>(t, f, nt, maps, err);
+  k_line<DIR, OP, TT, RS, V><<<grid, kLanes, smem, st>>>(t, f, nt, maps, err);
 }
 template <int DIR, int OP, class TT, class RS = float>
 void launch_line2_t(int grid, size_t smem, cudaStream_t st, const LineTask* t, const int* f, int nt,
@@ -3417,9 +2907,9 @@ template <int DIR, int OP, class TT, class RS = float>
 cudaError_t line2_smem_limit(int bytes) {
   return cudaFuncSetAttribute(k_line2<DIR, OP, TT, RS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
-template <int DIR, int OP, class TT, class RS>
+template <int DIR, int OP, class TT, class RS, int V>
 cudaError_t line_smem_limit(int bytes) {
-  return cudaFuncSetAttribute(k_line<DIR, OP, TT, RS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  return cudaFuncSetAttribute(k_line<DIR, OP, TT, RS, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
 }  // namespace canard

@@ -98,18 +98,25 @@ CANARD_QUAD_LINE(1, float)
 CANARD_QUAD_LINE(2, float)
 CANARD_QUAD_LINE(3, float)
 #undef CANARD_QUAD_LINE
-// one-lane sweeps with an FP32 elimination (the autotuner's alternative)
-#define CANARD_F32_LINE1(DIR, OP, TT)                                                                         \
-  CANARD_F32_EXTERN template void launch_line_t<DIR, OP, TT, float>(int, size_t, cudaStream_t, const LineTask*, \
+// one-lane sweeps with contraction: FP32 derivatives, the filter of the FP64
+// state with an FP32 elimination, and both in FP64 (the fast mode)
+#define CANARD_FMA_LINE1(DIR, OP, TT, RS)                                                                       \
+  CANARD_F32_EXTERN template void launch_line_t<DIR, OP, TT, RS, 1>(int, size_t, cudaStream_t, const LineTask*, \
                                                                     const int*, int, const CUtensorMap*, int*); \
-  CANARD_F32_EXTERN template cudaError_t line_smem_limit<DIR, OP, TT, float>(int);
-CANARD_F32_LINE1(1, 0, float)
-CANARD_F32_LINE1(2, 0, float)
-CANARD_F32_LINE1(3, 0, float)
-CANARD_F32_LINE1(1, 1, double)
-CANARD_F32_LINE1(2, 1, double)
-CANARD_F32_LINE1(3, 1, double)
-#undef CANARD_F32_LINE1
+  CANARD_F32_EXTERN template cudaError_t line_smem_limit<DIR, OP, TT, RS, 1>(int);
+CANARD_FMA_LINE1(1, 0, float, float)
+CANARD_FMA_LINE1(2, 0, float, float)
+CANARD_FMA_LINE1(3, 0, float, float)
+CANARD_FMA_LINE1(1, 1, double, float)
+CANARD_FMA_LINE1(2, 1, double, float)
+CANARD_FMA_LINE1(3, 1, double, float)
+CANARD_FMA_LINE1(1, 0, double, double)
+CANARD_FMA_LINE1(2, 0, double, double)
+CANARD_FMA_LINE1(3, 0, double, double)
+CANARD_FMA_LINE1(1, 1, double, double)
+CANARD_FMA_LINE1(2, 1, double, double)
+CANARD_FMA_LINE1(3, 1, double, double)
+#undef CANARD_FMA_LINE1
 // the filter of the FP64 state streamed into FP32 right-hand sides (split FP32 solve)
 #define CANARD_F32_FILT(DIR)                                                                              \
   CANARD_F32_EXTERN template void launch_filt2s_t<DIR>(int, size_t, cudaStream_t, const LineTask*, const int*, \

@@ -13,7 +13,7 @@
 // Results leave by coalesced stores (32 consecutive x per row).
 //
 // Every row is evaluated with the same operations in the same order as
-// sweep_deriv / sweep_filter (src/mo_numerics.f90:742-792, 922-977), so the
+// sweep_line (src/mo_numerics.f90:742-792, 922-977), so the
 // results are bit-identical to k_line's.
 #pragma once
 #include "kernels.cuh"
@@ -41,6 +41,21 @@ constexpr size_t kTmSmem = kTmHeader + kTmWarps * kTmWarpDoubles * sizeof(double
 #else
 #define TM_TRACE(k)
 #endif
+
+// The factors of a line: the interior constants of rows [c0, c1] and the tables.
+template <class RS>
+struct LuRows {
+  const RS* __restrict__ l1;
+  const RS* __restrict__ l2;
+  const RS* __restrict__ u1;
+  const RS* __restrict__ u2;
+  const RS* __restrict__ u3;
+  RS cl1, cl2, cu1, cu2, cu3;
+  int c0, c1;
+  __device__ __forceinline__ LuRows(const RS* lu, int L, RS a, RS b, RS c, RS d, RS e, int c0_)
+      : l1(lu), l2(lu + L), u1(lu + 2 * L), u2(lu + 3 * L), u3(lu + 4 * L), cl1(a), cl2(b), cu1(c), cu2(d),
+        cu3(e), c0(c0_), c1(L - 4) {}
+};
 
 // TMEM is not memory the compiler tracks: no "memory" clobbers, so shared and
 // global accesses can be scheduled across these; the tcgen05 statements stay
