@@ -312,17 +312,15 @@ struct BlockState {
   BlockGeom g;
   double* arena = nullptr;
   double* qb = nullptr;  // time-averaged recording (5 fields, padded rows), while recording is on
-  BlockDev dev;  // host copy of the device descriptor
+  BlockDev dev{};  // host copy of the device descriptor
   double *lu[2][3] = {};       // [nt][dir]: 5 * L
   double luc[2][3][5] = {};    // bitwise-constant interior factors
   int luc0[2][3] = {};         // first row of the constant range [luc0, L-4]
   double *recv[2][3] = {};     // [nt][dir]: 5 fields x 2 sides x ncomp x nbs
   double* chain[3] = {};       // [dir]: 2 sides x nbs
   double* drva[3] = {};        // (nbs,5,0:1)
-  double* drvb[3] = {};
   double* cm[3] = {};          // (nbs,3,0:1)
-  long long* gc_pts = nullptr;
-  double* gc_w = nullptr;
+  unsigned char* forced = nullptr;  // BlockDev::forced
   std::vector<GcbcFace> gc_faces;
   long long* sp_pts = nullptr;
   double *sp_a = nullptr, *sp_b = nullptr;
@@ -336,7 +334,6 @@ struct BlockState {
   int luc032[2][3] = {};      // first row of that range
   float* recv32[3] = {};  // derivative receive buffers of the FP32 fields
   float* drva32[3] = {};
-  float* drvb32[3] = {};
   // FP64 factors (5 L) followed by the FP64 split-solve tables (4 (L + 8)):
   // the fast FP64 mode's line kind, also a filter candidate of the mixed path
   double* lu64s[2][3] = {};
@@ -429,11 +426,10 @@ struct canard_ctx {
   // (kind < 0: the precision's default); set by canard_autotune
   struct TuneChoice { int kind = -1; int nc = 0; } tune[3][3];
   Table<FaceTask> mp_filt[5][3], mp_visc, mp_flux;
-  Table<GcbcTask> gc_setup, gc_upd[3][2];
-  void** fc_src = nullptr;
-  void** fc_dst = nullptr;
-  int* fc_cnt = nullptr;
-  int fc_n = 0, fc_max = 0;
+  Table<GcbcTask> gcbc;      // every GCBC face, block by block in the reference's face order
+  bool gc_curved = false;    // some face is a curved interface
+  void* gc_dh = nullptr;     // GcbcTask::dh of all faces
+  ForcedPts forced{};        // the points GCBC and sponge change
   Table<SpongeTask> sponge;
   AvgDev avg_pt, avg_ln, avg_sf;
   // union of the three plans' target points: the primitives are recomputed
@@ -441,9 +437,8 @@ struct canard_ctx {
   int prim_n = 0;
   int* prim_tb = nullptr;
   long long* prim_tl = nullptr;
-  // step-path fusions: flux sum inside the RK update (no GCBC, no sponge in
-  // the context), next stage's primitives inside the RK update
-  bool fuse_sum = false, fuse_prim = true;
+  // step-path fusion: next stage's primitives inside the RK update
+  bool fuse_prim = true;
   // wall_condition_update: wall-face points, packed reset kinds (k_wall_update)
   double* dtsum = nullptr;  // [ncases] recording interval, while recording is on
   // every block-face point (k_rk_faces)
@@ -1223,39 +1218,33 @@ void ph_visc_fluxes(canard_ctx* c, const StageParams* sp) {
     else launch_flux_visc<double>(ew_grid(c), c->st, c->dbd, sp, c->dcc);
     CK(cudaGetLastError());
   }
-  flux_derivatives(c, !c->fuse_sum);
+  flux_derivatives(c, false);  // the RK update forms the sum
 }
 
-void ph_gcbc(canard_ctx* c, const StageParams* sp) {
-  if (c->gc_setup.ntasks == 0) return;
-  const int thr = 128;
-  auto grid = [](int n) { return std::max(1, std::min((n + 127) / 128, 148 * 8)); };
-  Timed tm(c, T_GCBC, 0.0);
-  (void)thr;
-  if (c->f32())
-    launch_gcbc_setup<float>(grid(c->gc_setup.total), c->st, c->dbd, c->gc_setup.tasks, c->gc_setup.first,
-                             c->gc_setup.ntasks, c->gc_setup.total, sp);
-  else
-    launch_gcbc_setup<double>(grid(c->gc_setup.total), c->st, c->dbd, c->gc_setup.tasks, c->gc_setup.first,
-                              c->gc_setup.ntasks, c->gc_setup.total, sp);
-  CK(cudaGetLastError());
-  for (int d = 0; d < 3; ++d)
-    for (int s = 0; s < 2; ++s) c->launches += c->gc_upd[d][s].ntasks > 0 ? 1 : 0;
-  if (c->fc_n > 0) {
+// gcbc_setup, gcbc_comm, gcbc_update (the phase of the C ABI); step: on the
+// step path, where the right-hand sides of the forced points are summed here
+// and the sponge follows in the same launch
+void ph_gcbc(canard_ctx* c, const StageParams* sp, bool step = false) {
+  const auto& T = c->gcbc;
+  const int np = c->forced.ng + (step ? c->forced.ns : 0);
+  if (np == 0) return;
+  auto grid = [](int n) { return std::max(1, std::min((n + 127) / 128, 148 * 16)); };
+  auto faces = [&](bool setup, bool change) {
     c->launches += 1;
-    const dim3 g(std::max(1, std::min((c->fc_max + 255) / 256, 1024)), c->fc_n);
-    if (c->f32()) launch_face_copy<float>(g, c->st, c->fc_src, c->fc_dst, c->fc_cnt, c->fc_n);
-    else launch_face_copy<double>(g, c->st, c->fc_src, c->fc_dst, c->fc_cnt, c->fc_n);
+    if (c->f32())
+      launch_gcbc_faces<float>(grid(T.total), c->st, c->dbd, T.tasks, T.first, T.ntasks, T.total, sp, setup, change, step);
+    else
+      launch_gcbc_faces<double>(grid(T.total), c->st, c->dbd, T.tasks, T.first, T.ntasks, T.total, sp, setup, change, step);
     CK(cudaGetLastError());
+  };
+  Timed tm(c, T_GCBC, 0.0);
+  if (T.ntasks > 0) {
+    faces(true, !c->gc_curved);
+    if (c->gc_curved) faces(false, true);
   }
-  for (int d = 0; d < 3; ++d)
-    for (int s = 0; s < 2; ++s) {
-      const auto& T = c->gc_upd[d][s];
-      if (T.ntasks == 0) continue;
-      if (c->f32()) launch_gcbc_update<float>(grid(T.total), c->st, c->dbd, T.tasks, T.first, T.ntasks, T.total, sp);
-      else launch_gcbc_update<double>(grid(T.total), c->st, c->dbd, T.tasks, T.first, T.ntasks, T.total, sp);
-      CK(cudaGetLastError());
-    }
+  if (c->f32()) launch_forced_points<float>(grid(np), c->st, c->dbd, T.tasks, T.first, T.ntasks, c->forced, step);
+  else launch_forced_points<double>(grid(np), c->st, c->dbd, T.tasks, T.first, T.ntasks, c->forced, step);
+  CK(cudaGetLastError());
 }
 
 void ph_sponge(canard_ctx* c) {
@@ -1280,15 +1269,15 @@ void ph_rk(canard_ctx* c, const StageParams* sp) {
 // context allows (k_rk_next)
 void ph_rk_next(canard_ctx* c, const StageParams* sp, bool prim) {
   // the last stage stores the summed right-hand side (readable after a step)
-  const int sum = c->fuse_sum ? (prim ? 1 : 2) : 0;
+  const int last = prim ? 0 : 1;
   // FP32 stages 1-3 without GCBC, sponge or walls: the stage state only on the
   // block faces (the FP32 fluxes read the primitives), stored by k_rk_faces;
   // worth it while the face points are few (large blocks)
-  const bool faces = c->f32() && prim && c->fuse_sum && c->wall_n == 0 && c->face_n > 0 &&
+  const bool faces = c->f32() && prim && c->forced.ng + c->forced.ns == 0 && c->wall_n == 0 && c->face_n > 0 &&
                      c->face_n < 0.05 * valid_points(c);
-  Timed tm(c, T_RK, ew_bytes(c, 11 - (faces ? 5 : 0), (sum ? 15 : 5) + (sum == 2 ? 5 : 0) + (prim ? 7 : 0)));
-  if (c->f32()) launch_rk_next<float>(ew_grid(c), c->st, c->dbd, sp, c->dcc, sum, prim, faces ? 0 : 1);
-  else launch_rk_next<double>(ew_grid(c), c->st, c->dbd, sp, c->dcc, sum, prim, 1);
+  Timed tm(c, T_RK, ew_bytes(c, 11 - (faces ? 5 : 0), 15 + (last ? 5 : 0) + (prim ? 7 : 0)));
+  if (c->f32()) launch_rk_next<float>(ew_grid(c), c->st, c->dbd, sp, c->dcc, last, prim, faces ? 0 : 1);
+  else launch_rk_next<double>(ew_grid(c), c->st, c->dbd, sp, c->dcc, last, prim, 1);
   CK(cudaGetLastError());
   if (faces) {
     c->launches += 1;
@@ -1375,8 +1364,7 @@ void step_body(canard_ctx* c) {
     const StageParams* sp = dev_slot(c, nk - 1);
     if (nk > 1 && !c->fuse_prim) ph_prim(c);
     ph_visc_fluxes(c, sp);
-    ph_gcbc(c, sp);
-    ph_sponge(c);
+    ph_gcbc(c, sp, true);  // and the sponge
     const bool prim = c->fuse_prim && nk < 4;
     ph_rk_next(c, sp, prim);
     ph_wall(c, sp);
@@ -1645,12 +1633,24 @@ void build_tables(canard_ctx* c) {
 void build_gcbc_sponge_avg(canard_ctx* c) {
   const int nb = nblk(c);
   // GCBC tables need yaco (reference layout) on the host
-  std::vector<GcbcTask> setup_tasks;
-  std::vector<GcbcTask> upd[3][2];
-  std::vector<void*> fsrc;
-  std::vector<void*> fdst;
-  std::vector<int> fcnt;
+  std::vector<GcbcTask> gc_tasks;
   std::vector<SpongeTask> sp_tasks;
+  // forced points, GCBC's first, then the sponge's others (ForcedPts)
+  struct Forced { int b; long long l; int n, line[3]; double w[3], sa, sb; bool sp; };
+  std::vector<Forced> gpts;
+  std::vector<int> fb;         // the sponge's other points
+  std::vector<long long> fl;
+  std::vector<double> fsa, fsb;
+  int gc_lines = 0;
+  auto partner = [&](int b, int d, int side) -> void* {  // drva of the face that faces (b, d, side)
+    for (const FaceLink& L : c->links)
+      if (L.dst_b == b && L.nn == d && L.dst_side == side) {
+        const BlockState& S = c->blocks[L.src_b];
+        const size_t off = (size_t)5 * L.src_side * S.g.nbs[d];
+        return c->f32() ? static_cast<void*>(S.drva32[d] + off) : static_cast<void*>(S.drva[d] + off);
+      }
+    return nullptr;
+  };
   for (int b = 0; b < nb; ++b) {
     BlockState& B = c->blocks[b];
     const BlockGeom& g = B.g;
@@ -1665,31 +1665,35 @@ void build_gcbc_sponge_avg(canard_ctx* c) {
     std::vector<int64_t> pts;
     std::vector<double> w;
     gcbc_tables(g, yref.data(), B.gc_faces, pts, w);
-    if (!pts.empty()) {
-      std::vector<long long> p2(pts.begin(), pts.end());
-      B.gc_pts = dupload(p2, c->st);
-      B.gc_w = dupload(w, c->st);
-    }
+    std::vector<int> at;  // entry of every stored point in gpts, -1: none
+    const size_t g0 = gpts.size();
+    if (!pts.empty()) at.assign((size_t)g.npad, -1);
     for (const GcbcFace& f : B.gc_faces) {
       const int d = f.nn - 1;
       GcbcTask t{};
       t.b = b; t.nn = f.nn; t.side = f.side; t.bc = f.bc;
       t.cm = B.cm[d] + (size_t)3 * f.side * g.nbs[d];
       const size_t off = (size_t)5 * f.side * g.nbs[d];
-      if (c->f32()) {
-        t.drva = B.drva32[d] + off;
-        t.drvb = (f.bc == BC_CURV) ? B.drvb32[d] + off : nullptr;
-      } else {
-        t.drva = B.drva[d] + off;
-        t.drvb = (f.bc == BC_CURV) ? B.drvb[d] + off : nullptr;
-      }
-      t.pts = B.gc_pts + f.first;
-      t.w = B.gc_w + f.first;
+      t.drva = c->f32() ? static_cast<void*>(B.drva32[d] + off) : static_cast<void*>(B.drva[d] + off);
+      t.drvb = f.bc == BC_CURV ? partner(b, d, f.side) : nullptr;
+      c->gc_curved = c->gc_curved || f.bc == BC_CURV;
       t.nbs = g.nbs[d];
       t.nj = g.ijk[1][d] + 1;
       t.X = g.X; t.Y = g.Y; t.Z = g.Z; t.Xp = g.Xp; t.N = g.ijk[0][d];
-      setup_tasks.push_back(t);
-      upd[d][f.side].push_back(t);
+      // the face's five layers of points, in face order: at most one face per direction reaches a point
+      for (int64_t e = 0; e < (int64_t)5 * t.nbs; ++e) {
+        int& k = at[(size_t)pts[f.first + e]];
+        if (k < 0) {
+          k = (int)gpts.size();
+          gpts.push_back({b, (long long)pts[f.first + e], 0, {-1, -1, -1}, {0, 0, 0}, 0, 0, false});
+        }
+        Forced& q = gpts[k];
+        if (q.n == 3) throw ApiError(CANARD_ERR_UNSUPPORTED, "a point within five layers of more than three faces");
+        q.line[q.n] = gc_lines + (int)(e / 5);
+        q.w[q.n++] = w[f.first + e];
+      }
+      gc_lines += t.nbs;
+      gc_tasks.push_back(t);
     }
     // sponge
     if (cs.d.szco != 0.0) {
@@ -1705,34 +1709,67 @@ void build_gcbc_sponge_avg(canard_ctx* c) {
         SpongeTask st{b, B.sp_pts, B.sp_a, B.sp_b, B.sp_n, 0};
         sp_tasks.push_back(st);
       }
+      for (size_t e = 0; e < sp.size(); ++e) {
+        const int k = at.empty() ? -1 : at[(size_t)sp[e]];
+        if (k >= 0) {
+          gpts[k].sp = true; gpts[k].sa = a[e]; gpts[k].sb = bb[e];
+        } else {
+          fb.push_back(b); fl.push_back((long long)sp[e]); fsa.push_back(a[e]); fsb.push_back(bb[e]);
+        }
+      }
+    }
+    // neighbouring entries at neighbouring points (the sponge's are)
+    std::vector<Forced> sorted;
+    sorted.reserve(gpts.size() - g0);
+    for (const int k : at)
+      if (k >= 0) sorted.push_back(gpts[k]);
+    std::copy(sorted.begin(), sorted.end(), gpts.begin() + g0);
+  }
+  const size_t es = c->f32() ? sizeof(float) : sizeof(double);
+  c->gc_dh = dalloc<char>((size_t)5 * gc_lines * es, c->st);
+  {
+    size_t off = 0;
+    for (GcbcTask& t : gc_tasks) {
+      t.dh = static_cast<char*>(c->gc_dh) + off;
+      off += (size_t)5 * t.nbs * es;
     }
   }
-  for (const FaceLink& L : c->links) {  // gcbc_comm: BC_INTER_CURV faces only
-    const BlockState& R = c->blocks[L.dst_b];
-    const BlockState& S = c->blocks[L.src_b];
-    const int d = L.nn;
-    if (R.g.nbc[d][L.dst_side] != BC_CURV) continue;
-    if (c->f32()) {
-      fsrc.push_back(S.drva32[d] + (size_t)5 * L.src_side * S.g.nbs[d]);
-      fdst.push_back(R.drvb32[d] + (size_t)5 * L.dst_side * R.g.nbs[d]);
-    } else {
-      fsrc.push_back(S.drva[d] + (size_t)5 * L.src_side * S.g.nbs[d]);
-      fdst.push_back(R.drvb[d] + (size_t)5 * L.dst_side * R.g.nbs[d]);
-    }
-    fcnt.push_back(5 * R.g.nbs[d]);
-  }
-  c->gc_setup = make_lines_table(c, setup_tasks, false, &GcbcTask::nbs, &GcbcTask::line0);
-  for (int d = 0; d < 3; ++d)
-    for (int s = 0; s < 2; ++s)
-      c->gc_upd[d][s] = make_lines_table(c, upd[d][s], false, &GcbcTask::nbs, &GcbcTask::line0);
-  c->fc_n = (int)fsrc.size();
-  if (c->fc_n) {
-    c->fc_src = dupload(fsrc, c->st);
-    c->fc_dst = dupload(fdst, c->st);
-    c->fc_cnt = dupload(fcnt, c->st);
-    c->fc_max = *std::max_element(fcnt.begin(), fcnt.end());
-  }
+  c->gcbc = make_lines_table(c, gc_tasks, false, &GcbcTask::nbs, &GcbcTask::line0);
   c->sponge = make_lines_table(c, sp_tasks, false, &SpongeTask::count, &SpongeTask::first);
+  if (!gpts.empty() || !fb.empty()) {
+    const size_t ng = gpts.size();
+    std::vector<int> pb(ng), ln(3 * ng);
+    std::vector<long long> pl(ng);
+    std::vector<double> sa(ng), sb(ng), pw(3 * ng);
+    std::vector<unsigned char> inside(ng);
+    std::vector<std::vector<unsigned char>> mask((size_t)nb);
+    for (int b = 0; b < nb; ++b) mask[(size_t)b].assign((size_t)c->blocks[b].g.npad, 0);
+    for (size_t e = 0; e < ng; ++e) {
+      const Forced& q = gpts[e];
+      pb[e] = q.b; pl[e] = q.l; sa[e] = q.sa; sb[e] = q.sb;
+      inside[e] = q.sp ? 1 : 0;
+      for (int k = 0; k < 3; ++k) { ln[k * ng + e] = q.line[k]; pw[k * ng + e] = q.w[k]; }
+    }
+    pb.insert(pb.end(), fb.begin(), fb.end());
+    pl.insert(pl.end(), fl.begin(), fl.end());
+    sa.insert(sa.end(), fsa.begin(), fsa.end());
+    sb.insert(sb.end(), fsb.begin(), fsb.end());
+    for (size_t e = 0; e < pb.size(); ++e) mask[(size_t)pb[e]][(size_t)pl[e]] = 1;
+    ForcedPts& F = c->forced;
+    F.b = dupload(pb, c->st); F.l = dupload(pl, c->st);
+    F.sa = dupload(sa, c->st); F.sb = dupload(sb, c->st);
+    F.line = dupload(ln, c->st); F.w = dupload(pw, c->st);
+    F.sponge = dupload(inside, c->st);
+    F.ng = (int)ng; F.ns = (int)fb.size();
+    std::vector<BlockDev> bdv;
+    for (int b = 0; b < nb; ++b) {
+      c->blocks[b].forced = dupload(mask[(size_t)b], c->st);
+      c->blocks[b].dev.forced = c->blocks[b].forced;
+      bdv.push_back(c->blocks[b].dev);
+    }
+    CK(cudaMemcpyAsync(c->dbd, bdv.data(), bdv.size() * sizeof(BlockDev), cudaMemcpyHostToDevice, c->st));
+    CK(cudaStreamSynchronize(c->st));
+  }
   // junction averaging plans (per case: blocks of one case only see each other)
   AvgPlan P, Lp, Sf;
   for (const CaseState& cs : c->cases) {
@@ -1838,7 +1875,6 @@ void build_gcbc_sponge_avg(canard_ctx* c) {
     c->prim_tb = dupload(pb, c->st);
     c->prim_tl = dupload(pl, c->st);
   }
-  c->fuse_sum = c->gc_setup.ntasks == 0 && c->sponge.total == 0;
 }
 
 // t_grid%grid_metrics on the device (src/mo_grid.f90:52-189)
@@ -1973,7 +2009,7 @@ void destroy(canard_ctx* c) {
     cudaFree(b.arena);
     for (int nt = 0; nt < 2; ++nt)
       for (int d = 0; d < 3; ++d) { cudaFree(b.lu[nt][d]); cudaFree(b.recv[nt][d]); }
-    for (int d = 0; d < 3; ++d) { cudaFree(b.chain[d]); cudaFree(b.drva[d]); cudaFree(b.drvb[d]); cudaFree(b.cm[d]); }
+    for (int d = 0; d < 3; ++d) { cudaFree(b.chain[d]); cudaFree(b.drva[d]); cudaFree(b.cm[d]); }
     cudaFree(b.arena32);
     for (int nt = 0; nt < 2; ++nt)
       for (int d = 0; d < 3; ++d) {
@@ -1982,8 +2018,8 @@ void destroy(canard_ctx* c) {
         cudaFree(b.lu64t[nt][d]);
         cudaFree(b.lu32t[nt][d]);
       }
-    for (int d = 0; d < 3; ++d) { cudaFree(b.recv32[d]); cudaFree(b.drva32[d]); cudaFree(b.drvb32[d]); }
-    cudaFree(b.gc_pts); cudaFree(b.gc_w); cudaFree(b.sp_pts); cudaFree(b.sp_a); cudaFree(b.sp_b);
+    for (int d = 0; d < 3; ++d) { cudaFree(b.recv32[d]); cudaFree(b.drva32[d]); }
+    cudaFree(b.forced); cudaFree(b.sp_pts); cudaFree(b.sp_a); cudaFree(b.sp_b);
   }
   for (auto& cs : c->cases) cudaFree(cs.dsch);
   cudaFree(c->dbd); cudaFree(c->dcc); cudaFree(c->dsp); cudaFree(c->ddt); cudaFree(c->derr);
@@ -1997,9 +2033,12 @@ void destroy(canard_ctx* c) {
   for (int d = 0; d < 3; ++d) { fl(c->filt5[d]); fl(c->visc[d]); fl(c->flux[d]); }
   for (int m = 0; m < 5; ++m) for (int i = 0; i < 3; ++i) { ft(c->filt[m][i]); ft(c->mp_filt[m][i]); }
   for (int d = 0; d < 3; ++d) { ft(c->filt5[d]); ft(c->mp_filt5[d]); ft(c->visc[d]); ft(c->flux[d]); }
-  ft(c->mp_visc); ft(c->mp_flux); ft(c->gc_setup); ft(c->sponge);
-  for (int d = 0; d < 3; ++d) for (int s = 0; s < 2; ++s) ft(c->gc_upd[d][s]);
-  cudaFree(c->fc_src); cudaFree(c->fc_dst); cudaFree(c->fc_cnt);
+  ft(c->mp_visc); ft(c->mp_flux); ft(c->gcbc); ft(c->sponge);
+  cudaFree(c->gc_dh);
+  for (const void* p : {(const void*)c->forced.b, (const void*)c->forced.l, (const void*)c->forced.sa,
+                        (const void*)c->forced.sb, (const void*)c->forced.line, (const void*)c->forced.w,
+                        (const void*)c->forced.sponge})
+    cudaFree(const_cast<void*>(p));
   cudaFree(c->prim_tb); cudaFree(c->prim_tl);
   cudaFree(c->wall_tb); cudaFree(c->wall_tl); cudaFree(c->wall_tk);
   cudaFree(c->dtsum);
@@ -2078,6 +2117,7 @@ void create(canard_ctx* c, const canard_case_desc* cases, int ncases, const cana
     d.xim = fptr(B, F_XIM); d.etm = fptr(B, F_ETM); d.zem = fptr(B, F_ZEM); d.yaco = fptr(B, F_YACO);
     d.tau = fptr(B, F_TAU); d.scr = fptr(B, F_SCR); d.xyz = fptr(B, F_XYZ);
     d.f = Work<float>{};
+    d.forced = nullptr;
     if (c->f32()) {
       B.arena32 = dalloc<float>((size_t)G_COUNT * g.npad, c->st);
       d.f.de = gptr(B, G_DE); d.f.p = gptr(B, G_P); d.f.mu = gptr(B, G_MU); d.f.tau = gptr(B, G_TAU);
@@ -2156,10 +2196,8 @@ void create(canard_ctx* c, const canard_case_desc* cases, int ncases, const cana
       if (c->f32()) {
         B.recv32[dir] = dalloc<float>((size_t)5 * 2 * 2 * nbs, c->st);
         B.drva32[dir] = dalloc<float>((size_t)10 * nbs, c->st);
-        B.drvb32[dir] = dalloc<float>((size_t)10 * nbs, c->st);
       }
       B.drva[dir] = dalloc<double>((size_t)10 * nbs, c->st);
-      B.drvb[dir] = dalloc<double>((size_t)10 * nbs, c->st);
       B.cm[dir] = dalloc<double>((size_t)6 * nbs, c->st);
     }
     bdv.push_back(d);

@@ -697,14 +697,19 @@ void sponge_list(const BlockGeom& g, const canard_case_desc& c, const double* xy
   pts.clear(); asz.clear(); bsz.clear();
   const int64_t L = (int64_t)g.X * g.Y * g.Z;
   const double ta = kPi / c.szth0, tb = kPi / c.szth1;
+  // outside the ramps the argument is clamped: most points need no cosine
+  const double cpi = std::cos(kPi);
+  auto ramp = [&](double r) {
+    const double v = std::fmax(std::fmin(r, kPi), 0.0);
+    return v == kPi ? cpi : v == 0.0 ? 1.0 : std::cos(v);
+  };
   for (int64_t l = 0; l < L; ++l) {
     const double x = xyz[l], y = xyz[l + L];
     const double r3 = 0.0 * y;
     const double r0 = ta * (x - ((r3 - c.doml0) + c.szth0));
     const double r1 = tb * (((r3 + c.doml1) - c.szth1) - x);
     // MIN/MAX return the non-NaN argument, as gfortran's do
-    const double c0 = std::cos(std::fmax(std::fmin(r0, kPi), 0.0));
-    const double c1 = std::cos(std::fmax(std::fmin(r1, kPi), 0.0));
+    const double c0 = ramp(r0), c1 = ramp(r1);
     const double d1 = (c.szco * 0.5) * ((2.0 + c0) + c1);
     const double d2 = (c.szco * 0.5) * (1.0 + c0);
     if (d1 > 1.0e-8) {

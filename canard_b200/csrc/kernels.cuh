@@ -68,6 +68,9 @@ struct BlockDev {
   // FP64: state, metric and Jacobian masters, and the FP64 work fields
   double *qa, *qo, *de, *p, *mu, *xim, *etm, *zem, *yaco, *tau, *scr, *xyz;
   Work<float> f;  // FP32 work fields and metric copies (mixed precision only)
+  // 1 at the points whose right-hand side the GCBC or the sponge changes (null:
+  // none in the block); one byte per stored point
+  const unsigned char* forced;
 };
 
 template <class R>
@@ -127,11 +130,23 @@ struct GcbcTask {  // one GCBC face of one block
   int b, nn, side, bc;
   const double* cm;       // cm(jk,3,side) base of this face side: [d][jk]
   void* drva;             // drva(jk,5,side): [c][jk], in the flux type
-  const void* drvb;
-  const long long* pts;   // 5 device indices per line
-  const double* w;        // 5 weights per line
+  const void* drvb;       // drva of the partner face (curved interfaces), else null
+  void* dh;               // the change of the conserved derivatives: [c][jk]
   int nbs, nj, line0;
   int X, Y, Z, Xp, N;
+};
+
+// The points whose right-hand side the GCBC changes (the first ng: up to three
+// faces reach a point, in the reference's face order) and the other points of
+// the sponge (ns of them).
+struct ForcedPts {
+  const int* b;            // [ng + ns] block
+  const long long* l;      // [ng + ns] point
+  const double *sa, *sb;   // [ng + ns] sponge coefficients
+  const int* line;         // [3][ng] line over all faces (GcbcTask::line0 + jk), -1: none
+  const double* w;         // [3][ng] weights
+  const unsigned char* sponge;  // [ng] the point also lies in the sponge
+  int ng, ns;
 };
 
 struct SpongeTask { int b; const long long* pts; const double* asz; const double* bsz; int count, first; };
@@ -2501,19 +2516,38 @@ __global__ void k_flux_sum(const BlockDev* __restrict__ bd) {
   }
 }
 
-// RK stage update of the step path, with two optional fusions: sum > 0 forms
-// de = sum of the three flux derivatives on the fly (no GCBC or sponge
-// changes de in between; sum == 2 also stores it, so that de holds the last
-// stage's right-hand side after a step), prim computes the next stage's
-// primitives from the new state. Same operations in the same order as k_flux_sum, k_rk and
-// k_prim, so bit-identical to running them one after the other. STORE_Q
+// the right-hand side of one point: stored (SUM false), or formed from the
+// three flux derivatives (src/mo_physics.f90:399)
+template <class R, bool SUM>
+__device__ __forceinline__ void rhs_of(const Work<R>& W, long long l, long long n, R dv[5]) {
+  if (SUM) {
+    R f[15];
+#pragma unroll
+    for (int k = 0; k < 15; ++k) f[k] = W.scr[l + k * n];
+#pragma unroll
+    for (int c = 0; c < 5; ++c) dv[c] = (f[3 * c] + f[3 * c + 1]) + f[3 * c + 2];
+  } else {
+#pragma unroll
+    for (int c = 0; c < 5; ++c) dv[c] = W.de[l + c * n];
+  }
+}
+
+// RK stage update of the step path. The right-hand side is the sum of the three
+// flux derivatives, formed on the fly, except at the points that GCBC or
+// sponge change (forced: k_forced_points has left it in de there); last (the
+// last stage) stores it everywhere, so that de holds it after a step; prim
+// computes the next stage's primitives from the new state. Same operations in
+// the same order as k_flux_sum, k_rk and k_prim, so bit-identical to running
+// them one after the other. With a separate sum for blocks with GCBC or sponge,
+// 160 bytes a point were written and read for the few percent of points that
+// change (4 x 193 x 129 x 65 points FP64: sum 153 us + update 182 us a stage). STORE_Q
 // false: the stage state is not stored (k_rk_faces stores it on the block
 // faces, the junction points); the FP32 fluxes of the next stage read the
 // primitives, and nothing else reads the interior state before the last stage
 // rewrites it.
 template <class R, bool STORE_Q = true>
 __global__ void k_rk_next(const BlockDev* __restrict__ bd, const StageParams* __restrict__ sp,
-                          const CaseConst* __restrict__ cc, int sum, int prim) {
+                          const CaseConst* __restrict__ cc, int last, int prim) {
   FOR_POINTS(bd[blockIdx.y]) {
     const Work<R> W = work<R>(B);
     const long long n = B.npad;
@@ -2523,23 +2557,14 @@ __global__ void k_rk_next(const BlockDev* __restrict__ bd, const StageParams* __
     // between two loads would hold the second behind the first's latency
     R dv[5];
     double qo[5];
-    if (sum) {
-      const R* r = W.scr;
-      R f[15];
-#pragma unroll
-      for (int k = 0; k < 15; ++k) f[k] = r[l + k * n];
-#pragma unroll
-      for (int c = 0; c < 5; ++c) dv[c] = (f[3 * c] + f[3 * c + 1]) + f[3 * c + 2];
-    } else {
-#pragma unroll
-      for (int c = 0; c < 5; ++c) dv[c] = W.de[l + c * n];
-    }
+    if (B.forced && B.forced[l]) rhs_of<R, false>(W, l, n, dv);
+    else rhs_of<R, true>(W, l, n, dv);
 #pragma unroll
     for (int c = 0; c < 5; ++c) qo[c] = B.qo[l + c * n];
     double q[5];
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
-      if (sum == 2) W.de[l + c * n] = dv[c];
+      if (last) W.de[l + c * n] = dv[c];
       q[c] = qo[c] - r1 * double(dv[c]);
       if (STORE_Q) B.qa[l + c * n] = q[c];
     }
@@ -2631,8 +2656,60 @@ __device__ __forceinline__ void r2q_apply(const Elem<R>& e, const R cm[3], const
   }
 }
 
+// sponge (src/mo_sponge.f90:75-88) at one point: the forcing is formed in FP64
+// from the FP64 state and added to the right-hand side in the flux type
 template <class R>
-__global__ void k_gcbc_setup(const BlockDev* __restrict__ bd, const GcbcTask* __restrict__ tasks,
+__device__ __forceinline__ void sponge_point(double a, double b, const double* __restrict__ qa, long long l, long long n,
+                                             R dv[5]) {
+  double q[5];
+#pragma unroll
+  for (int c = 0; c < 5; ++c) q[c] = qa[l + c * n];
+  dv[0] = R(double(dv[0]) + a * (q[0] - 1.0));
+#pragma unroll
+  for (int d = 1; d <= 3; ++d) dv[d] = R(double(dv[d]) + b * (q[d] - 0.0));
+  dv[4] = R(double(dv[4]) + a * (q[4] - (1.0 / kGam) * (1.0 / KGAMM1)));
+}
+
+// gcbc_update at one face point (src/mo_gcbc.f90:222-320): the wave amplitudes
+// the boundary replaces and the change of the conserved derivatives they make.
+// drv: this face's amplitudes, drvb: the partner's (curved interfaces)
+template <class R>
+__device__ __forceinline__ void gcbc_change(const GcbcTask& T, const StageParams& S, const Elem<R>& e, const R cm[3],
+                                            R q1, const R drv[5], const R* drvb, int jk) {
+  const R ra0 = R(1 - 2 * T.side);
+  R cha[5], dha[5];
+  for (int c = 0; c < 5; ++c) {
+    cha[c] = drv[c];
+    dha[c] = drvb ? drvb[(long long)c * T.nbs + jk] : R(0);
+  }
+  if (T.bc == 10) {
+    if (ra0 * ((e.vn + e.vs) + e.ao) > R(0)) cha[3] = 0;
+    if (ra0 * ((e.vn + e.vs) - e.ao) > R(0)) cha[4] = 0;
+  } else if (T.bc == 20 || T.bc == 25) {
+    const R dtwi = R(1.0 / (4 * S.dt + 1.0e-8));
+    R sd = 0;
+    for (int d = 0; d < 3; ++d) sd = sd + cm[d] * R(S.dudtmf[d]);
+    cha[3 + T.side] = cha[4 - T.side] + (((R(2) * ra0) * e.aoi) * q1) * (sd + dtwi * (e.vn + e.vs));
+  } else {
+    if (ra0 * (e.vn + e.vs) > R(0)) { cha[0] = dha[0]; cha[1] = dha[1]; cha[2] = dha[2]; }
+    if (ra0 * ((e.vn + e.vs) + e.ao) > R(0)) cha[3] = dha[3];
+    if (ra0 * ((e.vn + e.vs) - e.ao) > R(0)) cha[4] = dha[4];
+  }
+  R v[5];
+  for (int c = 0; c < 5; ++c) v[c] = cha[c] - drv[c];
+  r2q_apply<R>(e, cm, v, dha);
+  R* dh = static_cast<R*>(T.dh);
+  for (int c = 0; c < 5; ++c) dh[(long long)c * T.nbs + jk] = dha[c];
+}
+
+// The face points of all GCBC faces. SETUP: gcbc_setup (the amplitudes into
+// drva; SUM: the right-hand side from the flux derivatives, which the step path
+// does not sum elsewhere at these points); CHANGE: gcbc_update's change into
+// dh. Both in one launch where no face is a curved interface; a curved one
+// needs the partner's amplitudes (gcbc_comm, src/mo_gcbc.f90:186-220, read in
+// place), so the change runs as a second launch there.
+template <class R, bool SETUP, bool CHANGE, bool SUM>
+__global__ void k_gcbc_faces(const BlockDev* __restrict__ bd, const GcbcTask* __restrict__ tasks,
                              const int* __restrict__ line0s, int ntasks, int nlines,
                              const StageParams* __restrict__ sp) {
   for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < nlines; g += gridDim.x * blockDim.x) {
@@ -2646,119 +2723,83 @@ __global__ void k_gcbc_setup(const BlockDev* __restrict__ bd, const GcbcTask* __
     const long long n = B.npad;
     const long long l = ((long long)z * B.Y + y) * B.Xp + x;
     const R cm[3] = {R(T.cm[jk]), R(T.cm[T.nbs + jk]), R(T.cm[2 * T.nbs + jk])};
-    const Elem<R> e =
-        eleme<R>(cm, R(B.qa[l]), R(B.qa[l + n]), R(B.qa[l + 2 * n]), R(B.qa[l + 3 * n]), W.p[l], S.umf);
-    const R ra0 = R(((20 - T.bc) * (25 - T.bc) * (30 - T.bc)) / 3000);
-    const R ra1 = R(1) - ra0;
-    R* drva = static_cast<R*>(T.drva);
-    R v[5], r[5];
-    for (int c = 0; c < 5; ++c) {
-      const R cha = ra0 * drva[(long long)c * T.nbs + jk] + ra1 * W.de[l + c * n];
-      v[c] = W.yaco[l] * cha;
-    }
-    q2r_apply<R>(e, cm, v, r);
-    for (int c = 0; c < 5; ++c) drva[(long long)c * T.nbs + jk] = r[c];
-  }
-}
-
-template <class R>
-__global__ void k_gcbc_update(const BlockDev* __restrict__ bd, const GcbcTask* __restrict__ tasks,
-                              const int* __restrict__ line0s, int ntasks, int nlines,
-                              const StageParams* __restrict__ sp) {
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < nlines; g += gridDim.x * blockDim.x) {
-    const GcbcTask& T = tasks[find_task(line0s, ntasks, g)];
-    const BlockDev& B = bd[T.b];
-    const Work<R> W = work<R>(B);
-    const StageParams S = sp[B.case_id];
-    const int jk = g - T.line0, j = jk % T.nj, k = jk / T.nj;
-    int x, y, z;
-    line_xyz(T.nn, T.side * T.N, j, k, x, y, z);
-    const long long n = B.npad;
-    const long long l = ((long long)z * B.Y + y) * B.Xp + x;
-    const R cm[3] = {R(T.cm[jk]), R(T.cm[T.nbs + jk]), R(T.cm[2 * T.nbs + jk])};
     const R q1 = R(B.qa[l]);
     const Elem<R> e = eleme<R>(cm, q1, R(B.qa[l + n]), R(B.qa[l + 2 * n]), R(B.qa[l + 3 * n]), W.p[l], S.umf);
-    const R ra0 = R(1 - 2 * T.side);
-    const R* drva = static_cast<const R*>(T.drva);
-    const R* drvb = static_cast<const R*>(T.drvb);
-    R cha[5], dha[5], drv[5];
-    for (int c = 0; c < 5; ++c) {
-      drv[c] = drva[(long long)c * T.nbs + jk];
-      cha[c] = drv[c];
-      dha[c] = drvb ? drvb[(long long)c * T.nbs + jk] : R(0);
-    }
-    if (T.bc == 10) {
-      if (ra0 * ((e.vn + e.vs) + e.ao) > R(0)) cha[3] = 0;
-      if (ra0 * ((e.vn + e.vs) - e.ao) > R(0)) cha[4] = 0;
-    } else if (T.bc == 20 || T.bc == 25) {
-      const R dtwi = R(1.0 / (4 * S.dt + 1.0e-8));
-      R sd = 0;
-      for (int d = 0; d < 3; ++d) sd = sd + cm[d] * R(S.dudtmf[d]);
-      cha[3 + T.side] = cha[4 - T.side] + (((R(2) * ra0) * e.aoi) * q1) * (sd + dtwi * (e.vn + e.vs));
+    R* drva = static_cast<R*>(T.drva);
+    R r[5];
+    if (SETUP) {
+      const R ra0 = R(((20 - T.bc) * (25 - T.bc) * (30 - T.bc)) / 3000);
+      const R ra1 = R(1) - ra0;
+      R v[5], de[5];
+      rhs_of<R, SUM>(W, l, n, de);
+      for (int c = 0; c < 5; ++c) {
+        const R cha = ra0 * drva[(long long)c * T.nbs + jk] + ra1 * de[c];
+        v[c] = W.yaco[l] * cha;
+      }
+      q2r_apply<R>(e, cm, v, r);
+      for (int c = 0; c < 5; ++c) drva[(long long)c * T.nbs + jk] = r[c];
     } else {
-      if (ra0 * (e.vn + e.vs) > R(0)) { cha[0] = dha[0]; cha[1] = dha[1]; cha[2] = dha[2]; }
-      if (ra0 * ((e.vn + e.vs) + e.ao) > R(0)) cha[3] = dha[3];
-      if (ra0 * ((e.vn + e.vs) - e.ao) > R(0)) cha[4] = dha[4];
+      for (int c = 0; c < 5; ++c) r[c] = drva[(long long)c * T.nbs + jk];
     }
-    R v[5];
-    for (int c = 0; c < 5; ++c) v[c] = cha[c] - drv[c];
-    r2q_apply<R>(e, cm, v, dha);
-    // the five points of the line are distinct: their 25 values load before
-    // any of them is stored (a store between two loads would make the second
-    // wait for the first's latency, since the compiler cannot tell they differ)
-    long long pts[5];
-    R ws[5], dv[5][5];
-#pragma unroll
-    for (int ii = 0; ii <= 4; ++ii) {
-      pts[ii] = T.pts[(long long)jk * 5 + ii];
-      ws[ii] = R(T.w[(long long)jk * 5 + ii]);
-    }
-#pragma unroll
-    for (int ii = 0; ii <= 4; ++ii)
-#pragma unroll
-      for (int c = 0; c < 5; ++c) dv[ii][c] = W.de[pts[ii] + c * n];
-#pragma unroll
-    for (int ii = 0; ii <= 4; ++ii)
-#pragma unroll
-      for (int c = 0; c < 5; ++c) W.de[pts[ii] + c * n] = dv[ii][c] + ws[ii] * dha[c];
+    if (CHANGE) gcbc_change<R>(T, S, e, cm, q1, r, static_cast<const R*>(T.drvb), jk);
   }
 }
 
-// sponge (src/mo_sponge.f90:75-88): the forcing is formed in FP64 from the
-// FP64 state and added to de in the flux type
+// gcbc_update's accumulation, gathered: every point that a face reaches adds
+// the faces' weighted changes in the reference's face order (one thread per
+// point, so faces that meet at an edge need no launch of their own). SUM (the
+// step path): the right-hand side is formed from the flux derivatives, the
+// sponge follows in the same pass, and the sponge's other points are handled
+// by the same launch; the RK update forms the sum itself everywhere else.
+// Five launches per stage (flux sum, two to six face updates, sponge) become
+// this one.
+template <class R, bool SUM>
+__global__ void k_forced_points(const BlockDev* __restrict__ bd, const GcbcTask* __restrict__ tasks,
+                                const int* __restrict__ line0s, int ntasks, const ForcedPts P) {
+  const int total = SUM ? P.ng + P.ns : P.ng;
+  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
+    const BlockDev& B = bd[P.b[g]];
+    const Work<R> W = work<R>(B);
+    const long long l = P.l[g], n = B.npad;
+    R dv[5];
+    rhs_of<R, SUM>(W, l, n, dv);
+    bool sponge = true;
+    if (g < P.ng) {
+      sponge = P.sponge[g] != 0;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const int ln = P.line[(long long)q * P.ng + g];
+        if (ln < 0) break;
+        const GcbcTask& T = tasks[find_task(line0s, ntasks, ln)];
+        const R ws = R(P.w[(long long)q * P.ng + g]);
+        const R* dh = static_cast<const R*>(T.dh);
+        const int jk = ln - T.line0;
+#pragma unroll
+        for (int c = 0; c < 5; ++c) dv[c] = dv[c] + ws * dh[(long long)c * T.nbs + jk];
+      }
+    }
+    if (SUM && sponge) sponge_point<R>(P.sa[g], P.sb[g], B.qa, l, n, dv);
+#pragma unroll
+    for (int c = 0; c < 5; ++c) W.de[l + c * n] = dv[c];
+  }
+}
+
+// the sponge as the phase of the C ABI
 template <class R>
 __global__ void k_sponge(const BlockDev* __restrict__ bd, const SpongeTask* __restrict__ tasks,
                          const int* __restrict__ first, int ntasks, int total) {
   for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
     const SpongeTask& T = tasks[find_task(first, ntasks, g)];
     const BlockDev& B = bd[T.b];
-    R* de = work<R>(B).de;
+    const Work<R> W = work<R>(B);
     const int e = g - T.first;
     const long long l = T.pts[e], n = B.npad;
-    const double a = T.asz[e], bb = T.bsz[e];
-    // every input before the first store (see k_rk_next)
     R dv[5];
-    double q[5];
+    rhs_of<R, false>(W, l, n, dv);
+    sponge_point<R>(T.asz[e], T.bsz[e], B.qa, l, n, dv);
 #pragma unroll
-    for (int c = 0; c < 5; ++c) {
-      dv[c] = de[l + c * n];
-      q[c] = B.qa[l + c * n];
-    }
-    de[l] = R(double(dv[0]) + a * (q[0] - 1.0));
-    for (int d = 1; d <= 3; ++d) de[l + d * n] = R(double(dv[d]) + bb * (q[d] - 0.0));
-    de[l + 4 * n] = R(double(dv[4]) + a * (q[4] - (1.0 / kGam) * (1.0 / KGAMM1)));
+    for (int c = 0; c < 5; ++c) W.de[l + c * n] = dv[c];
   }
-}
-
-// drvb <- drva of the partner face (gcbc_comm, src/mo_gcbc.f90:186-220)
-template <class R>
-__global__ void k_face_copy(const void* const* __restrict__ src, void* const* __restrict__ dst,
-                            const int* __restrict__ counts, int nfaces) {
-  const int f = blockIdx.y;
-  if (f >= nfaces) return;
-  const R* s = static_cast<const R*>(src[f]);
-  R* d = static_cast<R*>(dst[f]);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < counts[f]; i += gridDim.x * blockDim.x) d[i] = s[i];
 }
 
 // ---------------------------------------------------------------------------
@@ -2825,10 +2866,10 @@ __global__ void k_rk_faces(const BlockDev* __restrict__ bd, const StageParams* _
   }
 }
 template <class R>
-void launch_rk_next(dim3 g, cudaStream_t st, const BlockDev* bd, const StageParams* sp, const CaseConst* cc, int sum,
+void launch_rk_next(dim3 g, cudaStream_t st, const BlockDev* bd, const StageParams* sp, const CaseConst* cc, int last,
                     int prim, int store_q) {
-  if (store_q) k_rk_next<R, true><<<g, 256, 0, st>>>(bd, sp, cc, sum, prim);
-  else k_rk_next<R, false><<<g, 256, 0, st>>>(bd, sp, cc, sum, prim);
+  if (store_q) k_rk_next<R, true><<<g, 256, 0, st>>>(bd, sp, cc, last, prim);
+  else k_rk_next<R, false><<<g, 256, 0, st>>>(bd, sp, cc, last, prim);
 }
 template <class R>
 void launch_rk_faces(int grid, cudaStream_t st, const BlockDev* bd, const StageParams* sp, const int* tb,
@@ -2844,24 +2885,26 @@ template <class R>
 void launch_rk(dim3 g, cudaStream_t st, const BlockDev* bd, const StageParams* sp) {
   k_rk<R><<<g, 256, 0, st>>>(bd, sp);
 }
+// setup / change: which parts of k_gcbc_faces; sum: on the step path
 template <class R>
-void launch_gcbc_setup(int grid, cudaStream_t st, const BlockDev* bd, const GcbcTask* t, const int* f, int nt,
-                       int total, const StageParams* sp) {
-  k_gcbc_setup<R><<<grid, 128, 0, st>>>(bd, t, f, nt, total, sp);
+void launch_gcbc_faces(int grid, cudaStream_t st, const BlockDev* bd, const GcbcTask* t, const int* f, int nt,
+                       int total, const StageParams* sp, bool setup, bool change, bool sum) {
+  if (setup && change && sum) k_gcbc_faces<R, true, true, true><<<grid, 128, 0, st>>>(bd, t, f, nt, total, sp);
+  else if (setup && change) k_gcbc_faces<R, true, true, false><<<grid, 128, 0, st>>>(bd, t, f, nt, total, sp);
+  else if (setup && sum) k_gcbc_faces<R, true, false, true><<<grid, 128, 0, st>>>(bd, t, f, nt, total, sp);
+  else if (setup) k_gcbc_faces<R, true, false, false><<<grid, 128, 0, st>>>(bd, t, f, nt, total, sp);
+  else k_gcbc_faces<R, false, true, false><<<grid, 128, 0, st>>>(bd, t, f, nt, total, sp);
 }
 template <class R>
-void launch_gcbc_update(int grid, cudaStream_t st, const BlockDev* bd, const GcbcTask* t, const int* f, int nt,
-                        int total, const StageParams* sp) {
-  k_gcbc_update<R><<<grid, 128, 0, st>>>(bd, t, f, nt, total, sp);
+void launch_forced_points(int grid, cudaStream_t st, const BlockDev* bd, const GcbcTask* t, const int* f, int nt,
+                          const ForcedPts& P, bool sum) {
+  if (sum) k_forced_points<R, true><<<grid, 128, 0, st>>>(bd, t, f, nt, P);
+  else k_forced_points<R, false><<<grid, 128, 0, st>>>(bd, t, f, nt, P);
 }
 template <class R>
 void launch_sponge(int grid, cudaStream_t st, const BlockDev* bd, const SpongeTask* t, const int* f, int nt,
                    int total) {
   k_sponge<R><<<grid, 256, 0, st>>>(bd, t, f, nt, total);
-}
-template <class R>
-void launch_face_copy(dim3 g, cudaStream_t st, const void* const* src, void* const* dst, const int* cnt, int n) {
-  k_face_copy<R><<<g, 256, 0, st>>>(src, dst, cnt, n);
 }
 template <class T>
 void launch_mpigo_t(int grid, cudaStream_t st, const FaceTask* t, const int* f, int nt, int total) {

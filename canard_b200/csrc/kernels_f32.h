@@ -30,14 +30,12 @@ CANARD_F32_EXTERN template void launch_rk_faces<float>(int, cudaStream_t, const 
                                                        const int*, const long long*, int);
 CANARD_F32_EXTERN template void launch_prim_points<float>(int, cudaStream_t, const BlockDev*, const CaseConst*,
                                                           const int*, const long long*, int);
-CANARD_F32_EXTERN template void launch_gcbc_setup<float>(int, cudaStream_t, const BlockDev*, const GcbcTask*,
-                                                         const int*, int, int, const StageParams*);
-CANARD_F32_EXTERN template void launch_gcbc_update<float>(int, cudaStream_t, const BlockDev*, const GcbcTask*,
-                                                          const int*, int, int, const StageParams*);
+CANARD_F32_EXTERN template void launch_gcbc_faces<float>(int, cudaStream_t, const BlockDev*, const GcbcTask*,
+                                                         const int*, int, int, const StageParams*, bool, bool, bool);
+CANARD_F32_EXTERN template void launch_forced_points<float>(int, cudaStream_t, const BlockDev*, const GcbcTask*,
+                                                            const int*, int, const ForcedPts&, bool);
 CANARD_F32_EXTERN template void launch_sponge<float>(int, cudaStream_t, const BlockDev*, const SpongeTask*,
                                                      const int*, int, int);
-CANARD_F32_EXTERN template void launch_face_copy<float>(dim3, cudaStream_t, const void* const*, void* const*,
-                                                        const int*, int);
 CANARD_F32_EXTERN template void launch_mpigo_t<float>(int, cudaStream_t, const FaceTask*, const int*, int, int);
 
 #define CANARD_F32_LINE(DIR, OP, TT)                                                                      \
