@@ -402,6 +402,11 @@ struct canard_ctx {
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   long long graph_launches[2] = {0, 0};
   bool use_graphs = true;
+  // while a step is captured: independent launches go on parallel branches of
+  // the graph (branch), through these streams, which never run work themselves
+  bool branching = false;
+  cudaStream_t side[2] = {nullptr, nullptr};
+  cudaEvent_t ev_fork = nullptr, ev_join[2] = {nullptr, nullptr};
   double* stage = nullptr;  // contiguous staging of host copies (reference layout)
   // canard_step_host: staging of every listed block's state and the two copy streams
   double* hs_stage = nullptr;
@@ -1121,11 +1126,26 @@ void ph_filter(canard_ctx* c) {
     }
     return;
   }
+  // A field's last sweep changes nothing the next field's contractions and
+  // sweeps read (the send chains advance in the contractions), so while a step
+  // is captured it runs on a branch of its own beside them.
+  cudaStream_t main = c->st;
   for (int m = 1; m <= 5; ++m)
     for (int inn = 1; inn <= 3; ++inn) {
       launch_mpigo(c, c->mp_filt[m - 1][inn - 1]);
+      const bool side = c->branching && inn == 3 && m < 5;
+      if (side) {
+        CK(cudaEventRecord(c->ev_fork, main));
+        CK(cudaStreamWaitEvent(c->side[0], c->ev_fork, 0));
+        c->st = c->side[0];
+      }
       launch_line(c, c->filt[m - 1][inn - 1], kNnf[inn - 1] - 1, 1);
+      c->st = main;
     }
+  if (c->branching) {
+    CK(cudaEventRecord(c->ev_join[0], c->side[0]));
+    CK(cudaStreamWaitEvent(main, c->ev_join[0], 0));
+  }
 }
 
 void ph_copyqo(canard_ctx* c) {
@@ -1154,21 +1174,57 @@ bool any_viscous(const canard_ctx* c) {
   return false;
 }
 
+// Three launches of at most this many tiles gain from running side by side
+// (about one wave each: 20 steps of TGV 64, 780 tiles a launch, 16.7 -> 15.6 ms);
+// larger ones take each other's cache lines (six 101 x 101 x 17 blocks, up to
+// 9700 tiles a launch, 41.2 ms in order and 42.4 side by side; four 193 x 129 x
+// 65 blocks 160.4 and 161.6).
+bool few_tiles(const Table<LineTask> (&T)[3]) {
+  int most = 0;
+  for (const auto& t : T) most = std::max(most, t.total);
+  return most <= 148 * 16;
+}
+
+// f(0), f(1), f(2): three groups of launches that neither read nor overwrite
+// what another of them writes. While a step is captured they become parallel
+// branches of the graph: a launch that does not fill the GPU runs beside the
+// others, and the last wave of one overlaps the next. Otherwise (phases, timers,
+// graphs off) they run in order.
+template <class Fn>
+void branch3(canard_ctx* c, bool small, Fn&& f) {
+  if (!c->branching || !small) {
+    for (int k = 0; k < 3; ++k) f(k);
+    return;
+  }
+  cudaStream_t main = c->st;
+  struct Restore {
+    canard_ctx* c;
+    cudaStream_t s;
+    ~Restore() { c->st = s; }
+  } restore{c, main};
+  CK(cudaEventRecord(c->ev_fork, main));
+  for (int k = 0; k < 2; ++k) {
+    CK(cudaStreamWaitEvent(c->side[k], c->ev_fork, 0));
+    c->st = c->side[k];
+    f(k);
+    CK(cudaEventRecord(c->ev_join[k], c->side[k]));
+  }
+  c->st = main;
+  f(2);
+  for (int k = 0; k < 2; ++k) CK(cudaStreamWaitEvent(main, c->ev_join[k], 0));
+}
+
 // interface contraction and the 12 derivative sweeps of u, v, w, T
 void viscous_gradients(canard_ctx* c) {
   launch_mpigo(c, c->mp_visc);
-  launch_line(c, c->visc[2], 2, 0);
-  launch_line(c, c->visc[1], 1, 0);
-  launch_line(c, c->visc[0], 0, 0);
+  branch3(c, few_tiles(c->visc), [&](int k) { launch_line(c, c->visc[2 - k], 2 - k, 0); });
 }
 
 // flux interface contraction, the 15 derivative sweeps and (unless the RK
 // update forms it) their sum into de
 void flux_derivatives(canard_ctx* c, bool sum = true) {
   launch_mpigo(c, c->mp_flux);
-  launch_line(c, c->flux[0], 0, 0);
-  launch_line(c, c->flux[1], 1, 0);
-  launch_line(c, c->flux[2], 2, 0);
+  branch3(c, few_tiles(c->flux), [&](int k) { launch_line(c, c->flux[k], k, 0); });
   if (!sum) return;
   Timed tm(c, T_FLUXSUM, ew_bytes(c, 0, 20));
   if (c->f32()) launch_flux_sum<float>(ew_grid(c), c->st, c->dbd);
@@ -1394,10 +1450,18 @@ void one_step(canard_ctx* c) {
     std::vector<long long> nsave;
     for (auto& cs : c->cases) nsave.push_back(cs.n);
     cudaGraph_t g = nullptr;
+    for (cudaStream_t& q : c->side)
+      if (!q) CK(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
+    for (cudaEvent_t* e : {&c->ev_fork, &c->ev_join[0], &c->ev_join[1]})
+      if (!*e) CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
     try {
+      c->branching = true;
       step_body(c);
+      c->branching = false;
     } catch (...) {
+      c->branching = false;
+      c->st = c->own;
       cudaStreamEndCapture(c->st, &g);
       if (g) cudaGraphDestroy(g);
       c->st = user;
@@ -2051,6 +2115,10 @@ void destroy(canard_ctx* c) {
   free_transient(c);
   cudaFree(c->hs_stage);
   if (c->s_in) cudaStreamDestroy(c->s_in);
+  for (cudaStream_t q : c->side)
+    if (q) cudaStreamDestroy(q);
+  for (cudaEvent_t e : {c->ev_fork, c->ev_join[0], c->ev_join[1]})
+    if (e) cudaEventDestroy(e);
   if (c->s_out) cudaStreamDestroy(c->s_out);
   if (c->own) cudaStreamDestroy(c->own);
 }
