@@ -368,13 +368,6 @@ const char* kTimerNames[T_NFAM] = {"deriv_xi", "deriv_eta", "deriv_zeta", "filte
                                    "mpigo", "primitives", "flux_components", "viscous_assemble", "flux_sum",
                                    "rk_update", "gcbc", "sponge", "averaging", "timestep", "copy_qo"};
 
-struct AvgDev {
-  int ntg = 0, nsrc = 0;
-  int *tb = nullptr, *tfirst = nullptr, *tcount = nullptr, *sb = nullptr;
-  long long *tl = nullptr, *sl = nullptr;
-  double* snap = nullptr;
-};
-
 }  // namespace
 
 struct canard_ctx {
@@ -436,12 +429,7 @@ struct canard_ctx {
   void* gc_dh = nullptr;     // GcbcTask::dh of all faces
   ForcedPts forced{};        // the points GCBC and sponge change
   Table<SpongeTask> sponge;
-  AvgDev avg_pt, avg_ln, avg_sf;
-  // union of the three plans' target points: the primitives are recomputed
-  // there after averaging when the RK update already formed them
-  int prim_n = 0;
-  int* prim_tb = nullptr;
-  long long* prim_tl = nullptr;
+  AvgDev avg;
   // step-path fusion: next stage's primitives inside the RK update
   bool fuse_prim = true;
   // wall_condition_update: wall-face points, packed reset kinds (k_wall_update)
@@ -1343,16 +1331,6 @@ void ph_rk_next(canard_ctx* c, const StageParams* sp, bool prim) {
   CK(cudaGetLastError());
 }
 
-// primitives at the averaged points (after ph_rk_next formed them everywhere)
-void ph_prim_points(canard_ctx* c) {
-  if (c->prim_n == 0) return;
-  Timed tm(c, T_PRIM, (8.0 * 5 + (c->f32() ? 4.0 : 8.0) * 7) * c->prim_n);
-  const int grid = std::max(1, std::min((c->prim_n + 255) / 256, 1184));
-  if (c->f32()) launch_prim_points<float>(grid, c->st, c->dbd, c->dcc, c->prim_tb, c->prim_tl, c->prim_n);
-  else launch_prim_points<double>(grid, c->st, c->dbd, c->dcc, c->prim_tb, c->prim_tl, c->prim_n);
-  CK(cudaGetLastError());
-}
-
 void ph_wall(canard_ctx* c, const StageParams* sp) {
   if (c->wall_n == 0) return;
   Timed tm(c, T_RK, 8.0 * 10 * c->wall_n);
@@ -1361,22 +1339,28 @@ void ph_wall(canard_ctx* c, const StageParams* sp) {
   CK(cudaGetLastError());
 }
 
-void run_avg(canard_ctx* c, const AvgDev& A, int mode) {
-  if (A.ntg == 0) return;
-  Timed tm(c, T_AVERAGE, 8.0 * 5 * (A.nsrc + A.ntg));
-  c->launches += 1;  // snapshot + combine
-  k_avg_snapshot<<<std::max(1, std::min((A.nsrc + 255) / 256, 1184)), 256, 0, c->st>>>(c->dbd, A.sb, A.sl,
-                                                                                       A.nsrc, A.snap);
+// average_point, average_line, average_surface; prim: then the primitives again
+// at the averaged and the wall points (ph_rk_next formed them everywhere before)
+void ph_average(canard_ctx* c, bool prim = false) {
+  const AvgDev& A = c->avg;
+  auto grid = [](int n) { return std::max(1, std::min((n + 127) / 128, 148 * 16)); };
+  if (A.n > 0) {
+    Timed tm(c, T_AVERAGE, 8.0 * 15 * A.n);
+    for (const AvgMeans* m : {&A.pt, &A.ln}) {
+      if (m->n == 0) continue;
+      c->launches += 1;
+      k_avg_mean<<<grid(m->n), 128, 0, c->st>>>(c->dbd, *m, A.pt.out);
+      CK(cudaGetLastError());
+    }
+    k_avg_faces<<<grid(A.n), 128, 0, c->st>>>(c->dbd, A);
+    CK(cudaGetLastError());
+  }
+  const int np = prim ? A.np : A.n;
+  if (np == 0) return;
+  Timed tm(c, T_AVERAGE, (8.0 * 10 + (prim ? 7 * (c->f32() ? 4.0 : 8.0) : 0)) * np);
+  if (c->f32()) launch_average_store<float>(grid(np), c->st, c->dbd, c->dcc, A, prim ? 1 : 0);
+  else launch_average_store<double>(grid(np), c->st, c->dbd, c->dcc, A, prim ? 1 : 0);
   CK(cudaGetLastError());
-  k_avg_combine<<<std::max(1, std::min((A.ntg + 255) / 256, 1184)), 256, 0, c->st>>>(
-      c->dbd, A.tb, A.tl, A.tfirst, A.tcount, A.ntg, A.snap, mode);
-  CK(cudaGetLastError());
-}
-
-void ph_average(canard_ctx* c) {
-  run_avg(c, c->avg_pt, 0);
-  run_avg(c, c->avg_ln, 0);
-  run_avg(c, c->avg_sf, 1);
 }
 
 bool needs_dt_reduction(const canard_ctx* c) {
@@ -1424,8 +1408,7 @@ void step_body(canard_ctx* c) {
     const bool prim = c->fuse_prim && nk < 4;
     ph_rk_next(c, sp, prim);
     ph_wall(c, sp);
-    ph_average(c);
-    if (prim) ph_prim_points(c);
+    ph_average(c, prim);
   }
   time_advance(c);
 }
@@ -1694,6 +1677,81 @@ void build_tables(canard_ctx* c) {
   }
 }
 
+// The averaging plans of all cases (AvgDev) and the points the walls reset,
+// whose primitives are redone with the averaged ones'.
+void build_average(canard_ctx* c, const AvgPlan& P, const AvgPlan& Lp, const AvgPlan& Sf,
+                   const std::map<std::pair<int, long long>, int>& wall) {
+  typedef std::pair<int, long long> Pt;
+  std::map<Pt, int> pt, ln;  // target index of a point
+  for (size_t k = 0; k < P.targets.size(); ++k) pt[{P.targets[k].b, (long long)P.targets[k].l}] = (int)k;
+  for (size_t k = 0; k < Lp.targets.size(); ++k) ln[{Lp.targets[k].b, (long long)Lp.targets[k].l}] = (int)k;
+  // a point as stored, after average_point, or after average_line
+  auto ref = [&](int b, long long l, int stage) {
+    AvgRef r{b, -1, l};
+    if (stage > 0) {
+      auto p = pt.find({b, l});
+      if (p != pt.end()) r.code = 2 * p->second;
+    }
+    if (stage > 1) {
+      auto q = ln.find({b, l});
+      if (q != ln.end()) r.code = 2 * q->second + 1;
+    }
+    return r;
+  };
+  auto refs = [&](const AvgPlan& p, int stage) {
+    std::vector<AvgRef> v;
+    for (size_t e = 0; e < p.src_b.size(); ++e) v.push_back(ref(p.src_b[e], (long long)p.src_l[e], stage));
+    return v;
+  };
+  auto means = [&](const AvgPlan& p, int stage, AvgMeans& m) {
+    m.n = (int)p.targets.size();
+    if (m.n == 0) return;
+    std::vector<int> f, n;
+    for (const AvgTarget& t : p.targets) { f.push_back(t.first); n.push_back(t.count); }
+    m.first = dupload(f, c->st);
+    m.count = dupload(n, c->st);
+    m.src = dupload(refs(p, stage), c->st);
+    m.out = dalloc<double>((size_t)5 * m.n, c->st);
+  };
+  AvgDev& A = c->avg;
+  means(P, 0, A.pt);
+  means(Lp, 1, A.ln);
+  A.src = dupload(refs(Sf, 2), c->st);
+  // the points of all three plans in memory order, each with average_surface's partners
+  std::vector<std::pair<Pt, int>> all;
+  all.reserve(Sf.targets.size());
+  for (size_t k = 0; k < Sf.targets.size(); ++k) all.push_back({{Sf.targets[k].b, (long long)Sf.targets[k].l}, (int)k});
+  std::sort(all.begin(), all.end());
+  std::vector<std::pair<Pt, int>> more;  // on an edge or corner, but on no averaged face
+  auto known = [&](const Pt& p) {
+    auto it = std::lower_bound(all.begin(), all.end(), std::make_pair(p, -1));
+    return it != all.end() && it->first == p;
+  };
+  for (const auto* m : {&pt, &ln})
+    for (const auto& e : *m)
+      if (!known(e.first)) more.push_back({e.first, -1});
+  std::sort(more.begin(), more.end());
+  more.erase(std::unique(more.begin(), more.end()), more.end());
+  all.insert(all.end(), more.begin(), more.end());
+  std::vector<AvgRef> own;
+  std::vector<int> first, count;
+  for (const auto& e : all) {
+    own.push_back(ref(e.first.first, e.first.second, 2));
+    first.push_back(e.second < 0 ? 0 : Sf.targets[e.second].first);
+    count.push_back(e.second < 0 ? 0 : Sf.targets[e.second].count);
+  }
+  A.n = (int)own.size();
+  auto averaged = [&](const Pt& p) { return known(p) || pt.count(p) || ln.count(p); };
+  for (const auto& e : wall)
+    if (!averaged(e.first)) own.push_back({e.first.first, -1, e.first.second});
+  A.np = (int)own.size();
+  A.own = dupload(own, c->st);
+  A.first = dupload(first, c->st);
+  A.count = dupload(count, c->st);
+  A.out = dalloc<double>((size_t)5 * A.n, c->st);
+  CK(cudaStreamSynchronize(c->st));
+}
+
 void build_gcbc_sponge_avg(canard_ctx* c) {
   const int nb = nblk(c);
   // GCBC tables need yaco (reference layout) on the host
@@ -1861,20 +1919,6 @@ void build_gcbc_sponge_avg(canard_ctx* c) {
     };
     append(P, p1); append(Lp, l1); append(Sf, s1);
   }
-  auto upload_avg = [&](const AvgPlan& p, AvgDev& A) {
-    A.ntg = (int)p.targets.size();
-    A.nsrc = (int)p.src_b.size();
-    if (A.ntg == 0) return;
-    std::vector<int> tb, tf, tc;
-    std::vector<long long> tl, sl(p.src_l.begin(), p.src_l.end());
-    for (const auto& t : p.targets) { tb.push_back(t.b); tl.push_back(t.l); tf.push_back(t.first); tc.push_back(t.count); }
-    A.tb = dupload(tb, c->st); A.tl = dupload(tl, c->st); A.tfirst = dupload(tf, c->st); A.tcount = dupload(tc, c->st);
-    A.sb = dupload(p.src_b, c->st); A.sl = dupload(sl, c->st);
-    A.snap = dalloc<double>((size_t)A.nsrc * 5, c->st);
-  };
-  upload_avg(P, c->avg_pt);
-  upload_avg(Lp, c->avg_ln);
-  upload_avg(Sf, c->avg_sf);
   // wall-face points with their resets in the reference's face order
   std::map<std::pair<int, long long>, int> wall;
   for (int b = 0; b < nb; ++b) {
@@ -1924,21 +1968,7 @@ void build_gcbc_sponge_avg(canard_ctx* c) {
       c->face_tl = dupload(fl, c->st);
     }
   }
-  // the primitives are recomputed at averaged and at reset wall points
-  std::vector<std::pair<int, long long>> pts;
-  for (const AvgPlan* p : {&P, &Lp, &Sf})
-    for (const auto& t : p->targets) pts.emplace_back(t.b, (long long)t.l);
-  for (const auto& e : wall) pts.push_back(e.first);
-  std::sort(pts.begin(), pts.end());
-  pts.erase(std::unique(pts.begin(), pts.end()), pts.end());
-  c->prim_n = (int)pts.size();
-  if (c->prim_n) {
-    std::vector<int> pb;
-    std::vector<long long> pl;
-    for (const auto& q : pts) { pb.push_back(q.first); pl.push_back(q.second); }
-    c->prim_tb = dupload(pb, c->st);
-    c->prim_tl = dupload(pl, c->st);
-  }
+  build_average(c, P, Lp, Sf, wall);
 }
 
 // t_grid%grid_metrics on the device (src/mo_grid.f90:52-189)
@@ -2103,14 +2133,17 @@ void destroy(canard_ctx* c) {
                         (const void*)c->forced.sb, (const void*)c->forced.line, (const void*)c->forced.w,
                         (const void*)c->forced.sponge})
     cudaFree(const_cast<void*>(p));
-  cudaFree(c->prim_tb); cudaFree(c->prim_tl);
   cudaFree(c->wall_tb); cudaFree(c->wall_tl); cudaFree(c->wall_tk);
   cudaFree(c->dtsum);
   cudaFree(c->face_tb); cudaFree(c->face_tl);
   for (auto& b : c->blocks) cudaFree(b.qb);
-  for (AvgDev* A : {&c->avg_pt, &c->avg_ln, &c->avg_sf}) {
-    cudaFree(A->tb); cudaFree(A->tl); cudaFree(A->tfirst); cudaFree(A->tcount); cudaFree(A->sb); cudaFree(A->sl);
-    cudaFree(A->snap);
+  {
+    const AvgDev& A = c->avg;
+    for (const void* p : {(const void*)A.own, (const void*)A.first, (const void*)A.count, (const void*)A.src,
+                          (const void*)A.pt.first, (const void*)A.pt.count, (const void*)A.pt.src,
+                          (const void*)A.pt.out, (const void*)A.ln.first, (const void*)A.ln.count,
+                          (const void*)A.ln.src, (const void*)A.ln.out, (const void*)A.out})
+      cudaFree(const_cast<void*>(p));
   }
   free_transient(c);
   cudaFree(c->hs_stage);

@@ -764,7 +764,7 @@ int case_plans(int32_t nranks, const canard_block_desc* ranks, int32_t nblocks, 
 }  // namespace
 
 // Junction averaging of one case on the host, through the plans the device
-// applies (k_avg_snapshot / k_avg_combine, same arithmetic in the same order):
+// applies (k_avg_mean, k_avg_faces: same arithmetic in the same order):
 // the check of the plan builder against the oracle without a GPU.
 extern "C" int canard_average_host(int32_t nranks, const canard_block_desc* ranks, int32_t nblocks,
                                    const int32_t* nbpc, const int32_t* mbcd, const int32_t* sub,

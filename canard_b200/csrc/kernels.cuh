@@ -2138,16 +2138,53 @@ __global__ void k_prim(const BlockDev* __restrict__ bd, const CaseConst* __restr
   }
 }
 
-// the primitives again at the points junction averaging changed (targets of
-// the three averaging plans), after a fused RK + primitives update
+// Junction averaging (average_point, average_line, average_surface: src/
+// mo_domdcomp.f90:439-559, src/mo_gcbc.f90:342-422). The three routines run one
+// after the other in the reference, each reading its partners' values as the
+// one before left them. Here the state stays as it is until all three are done:
+// k_avg_mean forms the points' means, then the lines' (reading a corner's mean
+// where the reference would), k_avg_faces the faces' running averages, and
+// k_average_store writes the results and redoes the primitives there. A
+// snapshot and a combination per routine plus the primitives took seven
+// launches a stage of 2-16 us each whatever the size; one launch that evaluated
+// edges on the spot took longer than all of them (dependent loads of the few
+// corner threads: 20 steps of TGV 64 15.6 -> 16.4 ms).
+struct AvgRef {   // a point of the state as one of the routines reads it
+  int b, code;    // code -1: as stored; 2k: average_point's result k; 2k+1: average_line's result k
+  long long l;
+};
+struct AvgMeans {  // average_point's or average_line's targets: means over src[first, first + count)
+  int n = 0;
+  const int *first = nullptr, *count = nullptr;
+  const AvgRef* src = nullptr;
+  double* out = nullptr;  // [n][5]
+};
+struct AvgDev {
+  int n = 0, np = 0;                 // averaged points; those and the points reset by walls
+  const AvgRef* own = nullptr;       // [np] the point, as average_surface finds it
+  const int *first = nullptr, *count = nullptr;  // [n] average_surface's partners in src
+  const AvgRef* src = nullptr;
+  AvgMeans pt, ln;
+  double* out = nullptr;             // [5][n]
+};
+
+// after averaging: the averaged values into the state, and (prim) the
+// primitives at those points and at the points reset by walls
 template <class R>
-__global__ void k_prim_points(const BlockDev* __restrict__ bd, const CaseConst* __restrict__ cc,
-                              const int* __restrict__ tb, const long long* __restrict__ tl, int ntg) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntg; t += gridDim.x * blockDim.x) {
-    const BlockDev& B = bd[tb[t]];
-    const long long l = tl[t], n = B.npad;
-    const double* q = B.qa;
-    prim_point<R>(work<R>(B), cc[B.case_id], l, n, q[l], q[l + n], q[l + 2 * n], q[l + 3 * n], q[l + 4 * n]);
+__global__ void k_average_store(const BlockDev* __restrict__ bd, const CaseConst* __restrict__ cc, const AvgDev A,
+                                int prim) {
+  const int total = prim ? A.np : A.n;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+    const BlockDev& B = bd[A.own[t].b];
+    const long long l = A.own[t].l, n = B.npad;
+    double q[5];
+#pragma unroll
+    for (int c = 0; c < 5; ++c) q[c] = t < A.n ? A.out[(long long)c * A.n + t] : B.qa[l + c * n];
+    if (t < A.n) {
+#pragma unroll
+      for (int c = 0; c < 5; ++c) B.qa[l + c * n] = q[c];
+    }
+    if (prim) prim_point<R>(work<R>(B), cc[B.case_id], l, n, q[0], q[1], q[2], q[3], q[4]);
   }
 }
 
@@ -2877,9 +2914,9 @@ void launch_rk_faces(int grid, cudaStream_t st, const BlockDev* bd, const StageP
   k_rk_faces<R><<<grid, 256, 0, st>>>(bd, sp, tb, tl, ntg);
 }
 template <class R>
-void launch_prim_points(int grid, cudaStream_t st, const BlockDev* bd, const CaseConst* cc, const int* tb,
-                        const long long* tl, int ntg) {
-  k_prim_points<R><<<grid, 256, 0, st>>>(bd, cc, tb, tl, ntg);
+void launch_average_store(int grid, cudaStream_t st, const BlockDev* bd, const CaseConst* cc, const AvgDev& A,
+                          int prim) {
+  k_average_store<R><<<grid, 128, 0, st>>>(bd, cc, A, prim);
 }
 template <class R>
 void launch_rk(dim3 g, cudaStream_t st, const BlockDev* bd, const StageParams* sp) {

@@ -28,8 +28,8 @@ CANARD_F32_EXTERN template void launch_rk_next<float>(dim3, cudaStream_t, const 
                                                       const CaseConst*, int, int, int);
 CANARD_F32_EXTERN template void launch_rk_faces<float>(int, cudaStream_t, const BlockDev*, const StageParams*,
                                                        const int*, const long long*, int);
-CANARD_F32_EXTERN template void launch_prim_points<float>(int, cudaStream_t, const BlockDev*, const CaseConst*,
-                                                          const int*, const long long*, int);
+CANARD_F32_EXTERN template void launch_average_store<float>(int, cudaStream_t, const BlockDev*, const CaseConst*,
+                                                            const AvgDev&, int);
 CANARD_F32_EXTERN template void launch_gcbc_faces<float>(int, cudaStream_t, const BlockDev*, const GcbcTask*,
                                                          const int*, int, int, const StageParams*, bool, bool, bool);
 CANARD_F32_EXTERN template void launch_forced_points<float>(int, cudaStream_t, const BlockDev*, const GcbcTask*,

@@ -75,46 +75,54 @@ __global__ void k_face_normals(const BlockDev* __restrict__ bd, const CmTask* __
   }
 }
 
-// junction / surface averaging: snapshot then ordered combination
-__global__ void k_avg_snapshot(const BlockDev* __restrict__ bd, const int* __restrict__ sb,
-                               const long long* __restrict__ sl, int nsrc, double* __restrict__ snap) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nsrc; e += gridDim.x * blockDim.x) {
-    const BlockDev& B = bd[sb[e]];
-    const long long l = sl[e];
-    for (int c = 0; c < 5; ++c) snap[(long long)e * 5 + c] = B.qa[l + c * B.npad];
+// Junction averaging, see AvgDev.
+__device__ __forceinline__ void avg_value(const BlockDev* __restrict__ bd, const double* __restrict__ pt,
+                                          const double* __restrict__ ln, const AvgRef& r, double q[5]) {
+  const BlockDev& B = bd[r.b];
+  const double* v = r.code < 0 ? B.qa + r.l : ((r.code & 1) ? ln : pt) + 5 * (r.code >> 1);
+  const long long st = r.code < 0 ? B.npad : 1;
+#pragma unroll
+  for (int c = 0; c < 5; ++c) q[c] = v[c * st];
+}
+// average_point / average_line: sum in the plan's order, then scale
+__global__ void k_avg_mean(const BlockDev* __restrict__ bd, const AvgMeans M, const double* __restrict__ pt) {
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < M.n; t += gridDim.x * blockDim.x) {
+    const int f = M.first[t], cnt = M.count[t];
+    double q[5];
+    for (int j0 = 0; j0 < cnt; j0 += 4) {  // four partners' loads in flight
+      double v[4][5];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (j0 + j < cnt) avg_value(bd, pt, nullptr, M.src[f + j0 + j], v[j]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (j0 + j < cnt) {
+#pragma unroll
+          for (int c = 0; c < 5; ++c) q[c] = j0 + j == 0 ? v[j][c] : q[c] + v[j][c];
+        }
+    }
+    const double s = 1.0 / (double)cnt;
+#pragma unroll
+    for (int c = 0; c < 5; ++c) M.out[5LL * t + c] = s * q[c];
   }
 }
-// mode 0: sum and scale (average_point / average_line); mode 1: running
-// average of average_surface.
-__global__ void k_avg_combine(const BlockDev* __restrict__ bd, const int* __restrict__ tb,
-                              const long long* __restrict__ tl, const int* __restrict__ tfirst,
-                              const int* __restrict__ tcount, int ntg, const double* __restrict__ snap, int mode) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntg; t += gridDim.x * blockDim.x) {
-    const BlockDev& B = bd[tb[t]];
-    const long long l = tl[t];
-    const int f = tfirst[t], cnt = tcount[t];
-    // all five components formed before any is stored (the stores cannot
-    // alias the snapshot, but the compiler cannot know that)
-    double out[5];
+// average_surface: the running average over the partners across the faces
+__global__ void k_avg_faces(const BlockDev* __restrict__ bd, const AvgDev A) {
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < A.n; t += gridDim.x * blockDim.x) {
+    const int f = A.first[t], cnt = A.count[t];
+    double q[5];
+    avg_value(bd, A.pt.out, A.ln.out, A.own[t], q);
+    double r1 = 1.0;
+    for (int j = 0; j < cnt; ++j) {
+      double v[5];
+      avg_value(bd, A.pt.out, A.ln.out, A.src[f + j], v);
+      r1 = r1 + 1.0;
+      const double r2 = 1.0 / r1;
 #pragma unroll
-    for (int c = 0; c < 5; ++c) {
-      if (mode == 0) {
-        double acc = snap[(long long)f * 5 + c];
-        for (int j = 1; j < cnt; ++j) acc = acc + snap[(long long)(f + j) * 5 + c];
-        out[c] = (1.0 / (double)cnt) * acc;
-      } else {
-        double q = B.qa[l + c * B.npad];
-        double r1 = 1.0;
-        for (int j = 0; j < cnt; ++j) {
-          r1 = r1 + 1.0;
-          const double r2 = 1.0 / r1;
-          q = r2 * ((r1 - 1.0) * q + snap[(long long)(f + j) * 5 + c]) + 0.0 * q;
-        }
-        out[c] = q;
-      }
+      for (int c = 0; c < 5; ++c) q[c] = r2 * ((r1 - 1.0) * q[c] + v[c]) + 0.0 * q[c];
     }
 #pragma unroll
-    for (int c = 0; c < 5; ++c) B.qa[l + c * B.npad] = out[c];
+    for (int c = 0; c < 5; ++c) A.out[(long long)c * A.n + t] = q[c];
   }
 }
 
