@@ -11,7 +11,10 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <atomic>
 #include <mutex>
+#include <system_error>
+#include <thread>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -405,6 +408,13 @@ struct canard_ctx {
   double* hs_stage = nullptr;
   size_t hs_n = 0;
   cudaStream_t s_in = nullptr, s_out = nullptr;
+  // copies of outputs into pageable host memory (copy_out): per worker thread a
+  // pinned chunk and a stream
+  static constexpr int kCopyWorkers = 8;
+  static constexpr size_t kCopyChunk = 2u << 20;
+  void* cp_pin[kCopyWorkers] = {};
+  cudaStream_t cp_st[kCopyWorkers] = {};
+  cudaEvent_t cp_ready = nullptr;
   size_t stage_n = 0;
   int* derr = nullptr;
   bool setup_done = false;
@@ -1685,9 +1695,14 @@ void build_average(canard_ctx* c, const AvgPlan& P, const AvgPlan& Lp, const Avg
   std::map<Pt, int> pt, ln;  // target index of a point
   for (size_t k = 0; k < P.targets.size(); ++k) pt[{P.targets[k].b, (long long)P.targets[k].l}] = (int)k;
   for (size_t k = 0; k < Lp.targets.size(); ++k) ln[{Lp.targets[k].b, (long long)Lp.targets[k].l}] = (int)k;
-  // a point as stored, after average_point, or after average_line
+  // a point as stored, after average_point, or after average_line; only points
+  // on a block edge can be targets of those two
   auto ref = [&](int b, long long l, int stage) {
     AvgRef r{b, -1, l};
+    const BlockGeom& g = c->blocks[b].g;
+    const int x = (int)(l % g.Xp), y = (int)(l / g.Xp % g.Y), z = (int)(l / ((long long)g.Xp * g.Y));
+    const int faces = (x == 0 || x == g.X - 1) + (y == 0 || y == g.Y - 1) + (z == 0 || z == g.Z - 1);
+    if (faces < 2) return r;
     if (stage > 0) {
       auto p = pt.find({b, l});
       if (p != pt.end()) r.code = 2 * p->second;
@@ -1700,6 +1715,7 @@ void build_average(canard_ctx* c, const AvgPlan& P, const AvgPlan& Lp, const Avg
   };
   auto refs = [&](const AvgPlan& p, int stage) {
     std::vector<AvgRef> v;
+    v.reserve(p.src_b.size());
     for (size_t e = 0; e < p.src_b.size(); ++e) v.push_back(ref(p.src_b[e], (long long)p.src_l[e], stage));
     return v;
   };
@@ -2073,6 +2089,59 @@ void d2h_field(canard_ctx* c, const BlockState& B, double* dst, const double* sr
   CK(cudaMemcpyAsync(dst, c->stage, n * sizeof(double), cudaMemcpyDeviceToHost, c->st));
 }
 
+// Copies a large output (written by work on c->st) into the caller's memory and
+// returns when it is there. A new pageable array costs a page fault per 4 KB
+// besides the copy, all on the thread that asks the driver for it (340 MB: 70
+// ms), so a few threads each move chunks through a pinned buffer of their own:
+// transfers, copies and faults of different chunks overlap. Small copies and
+// pinned arrays go straight.
+void copy_out(canard_ctx* c, void* dst, const void* src, size_t bytes) {
+  constexpr size_t chunk = canard_ctx::kCopyChunk;
+  const size_t chunks = (bytes + chunk - 1) / chunk;
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, dst) != cudaSuccess) {
+    cudaGetLastError();
+    at.type = cudaMemoryTypeUnregistered;
+  }
+  const int workers = (int)std::min<size_t>(std::min<size_t>(canard_ctx::kCopyWorkers, chunks),
+                                            std::max(1u, std::thread::hardware_concurrency()));
+  if (workers < 2 || at.type != cudaMemoryTypeUnregistered) {
+    CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, c->st));
+    CK(cudaStreamSynchronize(c->st));
+    return;
+  }
+  int dev = 0;
+  CK(cudaGetDevice(&dev));
+  if (!c->cp_ready) CK(cudaEventCreateWithFlags(&c->cp_ready, cudaEventDisableTiming));
+  for (int w = 0; w < workers; ++w) {
+    if (!c->cp_pin[w]) CK(cudaMallocHost(&c->cp_pin[w], chunk));
+    if (!c->cp_st[w]) CK(cudaStreamCreateWithFlags(&c->cp_st[w], cudaStreamNonBlocking));
+  }
+  CK(cudaEventRecord(c->cp_ready, c->st));
+  std::atomic<size_t> next{0};
+  std::atomic<int> failed{0};
+  auto work = [&](int w) {
+    cudaError_t e = cudaSetDevice(dev);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(c->cp_st[w], c->cp_ready, 0);
+    for (size_t k; e == cudaSuccess && (k = next.fetch_add(1)) < chunks;) {
+      const size_t off = k * chunk, n = std::min(chunk, bytes - off);
+      e = cudaMemcpyAsync(c->cp_pin[w], static_cast<const char*>(src) + off, n, cudaMemcpyDeviceToHost, c->cp_st[w]);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(c->cp_st[w]);
+      if (e == cudaSuccess) std::memcpy(static_cast<char*>(dst) + off, c->cp_pin[w], n);
+    }
+    if (e != cudaSuccess) failed.store((int)e);
+  };
+  std::vector<std::thread> pool;
+  try {
+    for (int w = 1; w < workers; ++w) pool.emplace_back(work, w);
+  } catch (const std::system_error&) {
+    // fewer threads than asked for: the ones there take the chunks
+  }
+  work(0);
+  for (auto& t : pool) t.join();
+  CK(static_cast<cudaError_t>(failed.load()));
+}
+
 int block_index(const canard_ctx* c, int icase, int iblock) {
   if (icase < 0 || icase >= (int)c->cases.size()) throw ApiError(CANARD_ERR_ARG, "case index out of range");
   const CaseState& cs = c->cases[icase];
@@ -2147,6 +2216,10 @@ void destroy(canard_ctx* c) {
   }
   free_transient(c);
   cudaFree(c->hs_stage);
+  for (void* q : c->cp_pin) cudaFreeHost(q);
+  for (cudaStream_t q : c->cp_st)
+    if (q) cudaStreamDestroy(q);
+  if (c->cp_ready) cudaEventDestroy(c->cp_ready);
   if (c->s_in) cudaStreamDestroy(c->s_in);
   for (cudaStream_t q : c->side)
     if (q) cudaStreamDestroy(q);
@@ -2219,6 +2292,7 @@ void create(canard_ctx* c, const canard_case_desc* cases, int ncases, const cana
     d.tau = fptr(B, F_TAU); d.scr = fptr(B, F_SCR); d.xyz = fptr(B, F_XYZ);
     d.f = Work<float>{};
     d.forced = nullptr;
+    d.qb = nullptr;
     if (c->f32()) {
       B.arena32 = dalloc<float>((size_t)G_COUNT * g.npad, c->st);
       d.f.de = gptr(B, G_DE); d.f.p = gptr(B, G_P); d.f.mu = gptr(B, G_MU); d.f.tau = gptr(B, G_TAU);
@@ -2765,19 +2839,24 @@ int canard_read_restart(canard_ctx* c, int32_t icase, int32_t iblock, const char
 int canard_record_enable(canard_ctx* c, int32_t on) {
   return guarded(c, [&] {
     CK(cudaStreamSynchronize(c->st));
+    std::vector<BlockDev> bdv;
+    if (on && c->dtsum) {  // on already: the averages start again in the same memory
+      for (auto& b : c->blocks) CK(cudaMemsetAsync(b.qb, 0, (size_t)5 * b.g.npad * sizeof(double), c->st));
+      CK(cudaMemsetAsync(c->dtsum, 0, c->cases.size() * sizeof(double), c->st));
+      CK(cudaStreamSynchronize(c->st));
+      return;
+    }
     for (auto& b : c->blocks) {
       cudaFree(b.qb);
       b.qb = nullptr;
+      if (on) b.qb = dalloc<double>((size_t)5 * b.g.npad, c->st);  // zeroed
+      b.dev.qb = b.qb;
+      bdv.push_back(b.dev);
     }
     cudaFree(c->dtsum);
     c->dtsum = nullptr;
-    if (!on) return;
-    for (auto& b : c->blocks) {
-      b.qb = dalloc<double>((size_t)5 * b.g.npad, c->st);
-      CK(cudaMemsetAsync(b.qb, 0, (size_t)5 * b.g.npad * sizeof(double), c->st));
-    }
-    c->dtsum = dalloc<double>(c->cases.size(), c->st);
-    CK(cudaMemsetAsync(c->dtsum, 0, c->cases.size() * sizeof(double), c->st));
+    CK(cudaMemcpyAsync(c->dbd, bdv.data(), bdv.size() * sizeof(BlockDev), cudaMemcpyHostToDevice, c->st));
+    if (on) c->dtsum = dalloc<double>(c->cases.size(), c->st);
     CK(cudaStreamSynchronize(c->st));
   });
 }
@@ -2785,16 +2864,9 @@ int canard_record_enable(canard_ctx* c, int32_t on) {
 int canard_record_accumulate(canard_ctx* c) {
   return guarded(c, [&] {
     if (!c->dtsum) throw ApiError(CANARD_ERR_STATE, "recording is off (canard_record_enable)");
-    for (auto& b : c->blocks) {
-      const long long n = 5 * b.g.npad;
-      const int grid = (int)std::max<long long>(1, std::min<long long>((n + 255) / 256, 148 * 8));
-      k_record_acc<<<grid, 256, 0, c->st>>>(b.qb, fptr(b, F_QO), fptr(b, F_QA), b.g.npad, b.g.X, b.g.Xp, c->dtime,
-                                            b.g.case_id);
-      CK(cudaGetLastError());
-    }
-    k_record_dtsum<<<(ncase(c) + 127) / 128, 128, 0, c->st>>>(c->dtsum, c->dtime, ncase(c));
+    k_record_acc<<<ew_grid(c), 256, 0, c->st>>>(c->dbd, c->dtime, c->dtsum);
     CK(cudaGetLastError());
-    c->launches += (long long)c->blocks.size() + 1;
+    c->launches += 1;
   });
 }
 
@@ -2803,14 +2875,10 @@ int canard_record_output(canard_ctx* c, int32_t icase, float* const* vart, doubl
     if (!c->dtsum) throw ApiError(CANARD_ERR_STATE, "recording is off (canard_record_enable)");
     if (!vart || icase < 0 || icase >= (int)c->cases.size()) throw ApiError(CANARD_ERR_ARG, "bad case / pointer");
     const CaseState& cs = c->cases[icase];
-    size_t most = 0;
-    for (int b = cs.b0; b < cs.b0 + cs.nb; ++b) {
+    for (int b = cs.b0; b < cs.b0 + cs.nb; ++b)
       if (!vart[b - cs.b0]) throw ApiError(CANARD_ERR_ARG, "null output array");
-      const BlockGeom& g = c->blocks[b].g;
-      most = std::max(most, (size_t)5 * g.X * g.Y * g.Z);
-    }
-    float* dout = dalloc<float>(most, c->st);
-    c->transient.push_back(dout);
+    // packed in the staging buffer of the host copies (5 doubles a point of the largest block)
+    float* dout = reinterpret_cast<float*>(c->stage);
     for (int b = cs.b0; b < cs.b0 + cs.nb; ++b) {
       const BlockState& B = c->blocks[b];
       const BlockGeom& g = B.g;
@@ -2818,8 +2886,7 @@ int canard_record_output(canard_ctx* c, int32_t icase, float* const* vart, doubl
       k_record_out<<<grid, 256, 0, c->st>>>(B.qb, fptr(B, F_QO), dout, g.X, g.Y, g.Z, g.Xp, g.npad, c->dtime,
                                             c->dtsum, dev_slot(c, 3), icase);
       CK(cudaGetLastError());
-      CK(cudaMemcpyAsync(vart[b - cs.b0], dout, (size_t)5 * g.X * g.Y * g.Z * sizeof(float),
-                         cudaMemcpyDeviceToHost, c->st));
+      copy_out(c, vart[b - cs.b0], dout, (size_t)5 * g.X * g.Y * g.Z * sizeof(float));
     }
     TimeDev d;
     double dts = 0;
@@ -2832,7 +2899,6 @@ int canard_record_output(canard_ctx* c, int32_t icase, float* const* vart, doubl
       CK(cudaMemsetAsync(c->blocks[b].qb, 0, (size_t)5 * c->blocks[b].g.npad * sizeof(double), c->st));
     CK(cudaMemsetAsync(c->dtsum + icase, 0, sizeof(double), c->st));
     CK(cudaStreamSynchronize(c->st));
-    free_transient(c);
   });
 }
 

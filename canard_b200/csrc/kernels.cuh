@@ -71,6 +71,7 @@ struct BlockDev {
   // 1 at the points whose right-hand side the GCBC or the sponge changes (null:
   // none in the block); one byte per stored point
   const unsigned char* forced;
+  double* qb;  // time-averaged recording (5 fields), while it is on
 };
 
 template <class R>

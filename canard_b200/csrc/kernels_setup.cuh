@@ -249,18 +249,22 @@ __global__ void k_stage_params(const TimeDev* __restrict__ td, const CaseConst* 
 }
 
 // Time-averaged recording (src/mo_canard_driver.f90:373-378): after each step
-// qb = qb + (dt/2)(qo + qa) over the stored points of one block, and dtsum += dt.
-__global__ void k_record_acc(double* __restrict__ qb, const double* __restrict__ qo,
-                             const double* __restrict__ qa, long long npad, int X, int Xp,
-                             const TimeDev* __restrict__ td, int icase) {
-  const double fctr = 0.5 * td[icase].dt;
-  for (long long l = blockIdx.x * (long long)blockDim.x + threadIdx.x; l < 5 * npad;
-       l += (long long)gridDim.x * blockDim.x)
-    if ((int)(l % Xp) < X) qb[l] = qb[l] + fctr * (qo[l] + qa[l]);
-}
-__global__ void k_record_dtsum(double* dtsum, const TimeDev* __restrict__ td, int ncases) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < ncases) dtsum[c] = dtsum[c] + td[c].dt;
+// qb = qb + (dt/2)(qo + qa) over the stored points, and dtsum += dt of every
+// case: one launch for all blocks (a launch per block cost a batch of 64 blocks
+// 65 launches a step).
+__global__ void k_record_acc(const BlockDev* __restrict__ bd, const TimeDev* __restrict__ td,
+                             double* __restrict__ dtsum) {
+  const int b = blockIdx.y, icase = bd[b].case_id;
+  const double dt = td[icase].dt, fctr = 0.5 * dt;
+  FOR_POINTS(bd[b]) {
+    const long long n = B.npad;
+    double v[5];
+#pragma unroll
+    for (int c = 0; c < 5; ++c) v[c] = B.qb[l + c * n] + fctr * (B.qo[l + c * n] + B.qa[l + c * n]);
+#pragma unroll
+    for (int c = 0; c < 5; ++c) B.qb[l + c * n] = v[c];
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0 && (b == 0 || bd[b - 1].case_id != icase)) dtsum[icase] = dtsum[icase] + dt;
 }
 
 // An output of the recording (src/mo_canard_driver.f90:379-402): the average
