@@ -78,6 +78,7 @@ struct Table {
   CUtensorMap* maps = nullptr;  // line tables: TMA descriptors (in, out) per task
   int kind = 0;  // line tables: a LineKind; face tables: 0 FP64 fields, 1 FP32 fields
   int tdiv = 0;  // line tables: tiles per task when every task has as many (the kernels divide), else 0
+  int most = 0;  // face tables: lines of the largest face
 };
 
 // Element types of a line launch: tile (field) type and elimination type.
@@ -1049,7 +1050,7 @@ Table<FaceTask> make_face_table(canard_ctx* c, std::vector<FaceTask> v, bool tra
   T.kind = kind;
   std::vector<int> first;
   int tot = 0;
-  for (auto& t : v) { t.line0 = tot; first.push_back(tot); tot += t.nbs; }
+  for (auto& t : v) { t.line0 = tot; first.push_back(tot); tot += t.nbs; T.most = std::max(T.most, t.nbs); }
   T.ntasks = (int)v.size();
   T.total = tot;
   T.bytes = (double)tot * (12 + (v.empty() ? 0 : (v[0].nt ? 3 : 2))) * (kind ? sizeof(float) : sizeof(double));
@@ -1061,12 +1062,14 @@ Table<FaceTask> make_face_table(canard_ctx* c, std::vector<FaceTask> v, bool tra
 
 void launch_mpigo(canard_ctx* c, const Table<FaceTask>& T) {
   if (T.ntasks == 0) return;
-  const int thr = 128;
-  const int grid = std::min((T.total + thr - 1) / thr, 148 * 16);
   Timed tm(c, T_MPIGO, T.bytes);
-  if (T.kind) launch_mpigo_t<float>(grid, c->st, T.tasks, T.first, T.ntasks, T.total);
-  else launch_mpigo_t<double>(grid, c->st, T.tasks, T.first, T.ntasks, T.total);
-  CK(cudaGetLastError());
+  // the grid's second dimension holds 65535 faces
+  for (int k = 0; k < T.ntasks; k += 65535) {
+    const int n = std::min(T.ntasks - k, 65535);
+    if (T.kind) launch_mpigo_t<float>(c->st, T.tasks + k, n, T.most);
+    else launch_mpigo_t<double>(c->st, T.tasks + k, n, T.most);
+    CK(cudaGetLastError());
+  }
 }
 
 dim3 ew_grid(const canard_ctx* c) {
@@ -1689,9 +1692,26 @@ void build_tables(canard_ctx* c) {
 
 // The averaging plans of all cases (AvgDev) and the points the walls reset,
 // whose primitives are redone with the averaged ones'.
-void build_average(canard_ctx* c, const AvgPlan& P, const AvgPlan& Lp, const AvgPlan& Sf,
+void build_average(canard_ctx* c, const AvgPlan& P, const AvgPlan& Lp0, const AvgPlan& Sf,
                    const std::map<std::pair<int, long long>, int>& wall) {
   typedef std::pair<int, long long> Pt;
+  // A line's mean over the point itself two or four times (an edge of a block
+  // that is periodic onto itself) is the point: x + x, then (2x + x) + x = 4x
+  // exactly, and the scaling is exact. Such targets fall away; eight copies (a
+  // corner) may round and stay.
+  AvgPlan Lk;
+  for (const AvgTarget& t : Lp0.targets) {
+    bool self = t.count == 1 || t.count == 2 || t.count == 4;
+    for (int j = 0; j < t.count; ++j)
+      self = self && Lp0.src_b[t.first + j] == t.b && Lp0.src_l[t.first + j] == t.l;
+    if (self) continue;
+    AvgTarget u = t;
+    u.first = (int)Lk.src_b.size();
+    Lk.src_b.insert(Lk.src_b.end(), Lp0.src_b.begin() + t.first, Lp0.src_b.begin() + t.first + t.count);
+    Lk.src_l.insert(Lk.src_l.end(), Lp0.src_l.begin() + t.first, Lp0.src_l.begin() + t.first + t.count);
+    Lk.targets.push_back(u);
+  }
+  const AvgPlan& Lp = Lk;
   std::map<Pt, int> pt, ln;  // target index of a point
   for (size_t k = 0; k < P.targets.size(); ++k) pt[{P.targets[k].b, (long long)P.targets[k].l}] = (int)k;
   for (size_t k = 0; k < Lp.targets.size(); ++k) ln[{Lp.targets[k].b, (long long)Lp.targets[k].l}] = (int)k;
@@ -3392,10 +3412,7 @@ extern "C" int canard_deriv_noalloc(const double* d_in, double* d_out, int32_t l
     CK(cudaMemcpyToSymbolAsync(g_noalloc_scratch, lu.data(), lu.size() * sizeof(double), kNaLu,
                                cudaMemcpyHostToDevice, st));
     if (nf) {
-      const int tot = nf * nbs;
-      launch_mpigo_t<double>(std::max(1, std::min((tot + 127) / 128, 148 * 16)), st,
-                             reinterpret_cast<const FaceTask*>(base + kNaFace),
-                             reinterpret_cast<const int*>(base + kNaIdx) + 1, nf, tot);
+      launch_mpigo_t<double>(st, reinterpret_cast<const FaceTask*>(base + kNaFace), nf, nbs);
       CK(cudaGetLastError());
     }
     const size_t smem = line_smem(dir, t, LK_F64);

@@ -2027,68 +2027,80 @@ __device__ __forceinline__ void line_xyz(int nn, int pos, int j, int k, int& x, 
 }
 
 // t_numerics%mpigo for a list of faces (src/mo_numerics.f90:429-565), in the
-// field type T.
+// field type T. blockIdx.y: face, so no thread searches for its task, and the
+// face's 24 coefficients go to shared memory while its values load: bound by
+// latency at every size (20 launches a step of the plain filter and the flux
+// contractions), it has two dependent loads instead of six. A face whose
+// direction is not exchanged by this call only advances its send chain, which
+// takes the first of the 12 values: the plain filter, which advances all three
+// directions' chains in each of its 15 calls, reads a third of the values.
 template <class T>
-__global__ void k_mpigo(const FaceTask* __restrict__ tasks, const int* __restrict__ line0s, int ntasks,
-                        int nlines) {
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < nlines; g += gridDim.x * blockDim.x) {
-    const int ti = find_task(line0s, ntasks, g);
-    const FaceTask& F = tasks[ti];
-    const T* src = static_cast<const T*>(F.src);
-    // eta faces run x fastest across threads so their reads coalesce; the
-    // other faces already do (zeta) or read 12 contiguous values (xi)
-    const int gl = g - F.line0;
-    int j, k, jk;
-    if (F.nn == 2) {
-      k = gl % F.X;
-      j = gl / F.X;
-      jk = j + F.nj * k;
-    } else {
-      jk = gl;
-      j = jk % F.nj;
-      k = jk / F.nj;
-    }
-    const int istart = F.sb * F.N, step = 1 - 2 * F.sb;
-    int x, y, z;
-    line_xyz(F.nn, istart, j, k, x, y, z);
-    const T resk = T(F.ra0k) * src[((long long)z * F.Y + y) * F.Xp + x];
-    const DevScheme* sc = F.sc;
-    const int nt = F.nt;
-    T t0 = 0, t1 = 0, sap0 = 0;
+__global__ void k_mpigo(const FaceTask* __restrict__ tasks) {
+  const FaceTask& F = tasks[blockIdx.y];
+  const int nbs = F.nbs, first = blockIdx.x * blockDim.x;
+  if (first >= nbs) return;
+  __shared__ T co[2][12];
+  const int nt = F.nt;
+  const DevScheme* sc = F.sc;
+  if (threadIdx.x < 24) co[threadIdx.x / 12][threadIdx.x % 12] = T(sc->pbco[nt][threadIdx.x / 12][threadIdx.x % 12]);
+  const int gl = first + threadIdx.x;
+  const bool has = gl < nbs, exch = F.exch != 0;
+  const T* src = static_cast<const T*>(F.src);
+  // eta faces run x fastest across threads so their reads coalesce; the
+  // other faces already do (zeta) or read 12 contiguous values (xi)
+  int j, k, jk;
+  if (F.nn == 2) {
+    k = gl % F.X;
+    j = gl / F.X;
+    jk = j + F.nj * k;
+  } else {
+    jk = gl;
+    j = jk % F.nj;
+    k = jk / F.nj;
+  }
+  const int step = 1 - 2 * F.sb;
+  int x, y, z;
+  line_xyz(F.nn, F.sb * F.N, j, k, x, y, z);
+  const long long l0 = ((long long)z * F.Y + y) * F.Xp + x;
+  const long long ls = (F.nn == 1 ? 1LL : F.nn == 2 ? (long long)F.Xp : (long long)F.Xp * F.Y) * step;
+  T v[12];
 #pragma unroll
-    for (int i = 0; i < 12; ++i) {
-      line_xyz(F.nn, istart + step * (i + F.iik), j, k, x, y, z);
-      const T v = src[((long long)z * F.Y + y) * F.Xp + x];
-      if (i == 0) sap0 = v;
-      t0 = t0 + T(sc->pbco[nt][0][i]) * v;
-      t1 = t1 + T(sc->pbco[nt][1][i]) * v;
-    }
-    T snd0 = t0 - resk * T(sc->pbcot[nt][0]);
-    T snd1 = t1 - resk * T(sc->pbcot[nt][1]);
-    T snd2 = 0;
-    if (nt == 1) {
-      if (F.chain) {
-        const T old = T(F.chain[jk]);
-        snd2 = old + ((sap0 - resk) - old);
-        F.chain[jk] = double(snd2);
-      } else {
-        snd2 = sap0 - resk;  // the chain's exact value, without its rounding
-      }
-    }
-    if (F.exch) {
-      T* recv = static_cast<T*>(F.recv);
-      if (F.corr) {  // receiver side is periodic and n45 = n45go
-        line_xyz(F.nn, (1 - F.sb) * F.NA, j, k, x, y, z);
-        const T f = static_cast<const T*>(F.dstf)[((long long)z * F.YA + y) * F.XpA + x];
-        snd0 = snd0 + f * T(sc->pbcot[nt][0]);
-        snd1 = snd1 + f * T(sc->pbcot[nt][1]);
-        if (nt == 1) snd2 = snd2 + f; else snd1 = snd1 + T(0) * f;
-      }
-      recv[jk] = snd0;
-      recv[F.nbs + jk] = snd1;
-      if (nt == 1) recv[2 * F.nbs + jk] = snd2;
+  for (int i = 0; i < 12; ++i) v[i] = has && (exch || i == 0) ? src[l0 + ls * (i + F.iik)] : T(0);
+  const T face = has ? src[l0] : T(0);
+  T old = 0;
+  if (has && nt == 1 && F.chain) old = T(F.chain[jk]);
+  __syncthreads();
+  if (!has) return;
+  const T resk = T(F.ra0k) * face;
+  T snd2 = 0;
+  if (nt == 1) {
+    if (F.chain) {
+      snd2 = old + ((v[0] - resk) - old);
+      F.chain[jk] = double(snd2);
+    } else {
+      snd2 = v[0] - resk;  // the chain's exact value, without its rounding
     }
   }
+  if (!exch) return;
+  T t0 = 0, t1 = 0;
+#pragma unroll
+  for (int i = 0; i < 12; ++i) {
+    t0 = t0 + co[0][i] * v[i];
+    t1 = t1 + co[1][i] * v[i];
+  }
+  T snd0 = t0 - resk * T(sc->pbcot[nt][0]);
+  T snd1 = t1 - resk * T(sc->pbcot[nt][1]);
+  T* recv = static_cast<T*>(F.recv);
+  if (F.corr) {  // receiver side is periodic and n45 = n45go
+    line_xyz(F.nn, (1 - F.sb) * F.NA, j, k, x, y, z);
+    const T f = static_cast<const T*>(F.dstf)[((long long)z * F.YA + y) * F.XpA + x];
+    snd0 = snd0 + f * T(sc->pbcot[nt][0]);
+    snd1 = snd1 + f * T(sc->pbcot[nt][1]);
+    if (nt == 1) snd2 = snd2 + f; else snd1 = snd1 + T(0) * f;
+  }
+  recv[jk] = snd0;
+  recv[nbs + jk] = snd1;
+  if (nt == 1) recv[2 * nbs + jk] = snd2;
 }
 
 // ---------------------------------------------------------------------------
@@ -2944,9 +2956,10 @@ void launch_sponge(int grid, cudaStream_t st, const BlockDev* bd, const SpongeTa
                    int total) {
   k_sponge<R><<<grid, 256, 0, st>>>(bd, t, f, nt, total);
 }
+// nt faces of at most `lines` lines each
 template <class T>
-void launch_mpigo_t(int grid, cudaStream_t st, const FaceTask* t, const int* f, int nt, int total) {
-  k_mpigo<T><<<grid, 128, 0, st>>>(t, f, nt, total);
+void launch_mpigo_t(cudaStream_t st, const FaceTask* t, int nt, int lines) {
+  k_mpigo<T><<<dim3((unsigned)((lines + 127) / 128), (unsigned)nt), 128, 0, st>>>(t);
 }
 template <int DIR, int OP, class TT, class RS, int V>
 void launch_line_t(int grid, size_t smem, cudaStream_t st, const LineTask* t, const int* f, int nt,

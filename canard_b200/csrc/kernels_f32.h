@@ -36,7 +36,7 @@ CANARD_F32_EXTERN template void launch_forced_points<float>(int, cudaStream_t, c
                                                             const int*, int, const ForcedPts&, bool);
 CANARD_F32_EXTERN template void launch_sponge<float>(int, cudaStream_t, const BlockDev*, const SpongeTask*,
                                                      const int*, int, int);
-CANARD_F32_EXTERN template void launch_mpigo_t<float>(int, cudaStream_t, const FaceTask*, const int*, int, int);
+CANARD_F32_EXTERN template void launch_mpigo_t<float>(cudaStream_t, const FaceTask*, int, int);
 
 #define CANARD_F32_LINE(DIR, OP, TT)                                                                      \
   CANARD_F32_EXTERN template void launch_line2_t<DIR, OP, TT>(int, size_t, cudaStream_t, const LineTask*,   \
