@@ -1333,8 +1333,9 @@ void ph_rk_next(canard_ctx* c, const StageParams* sp, bool prim) {
   const bool faces = c->f32() && prim && c->forced.ng + c->forced.ns == 0 && c->wall_n == 0 && c->face_n > 0 &&
                      c->face_n < 0.05 * valid_points(c);
   Timed tm(c, T_RK, ew_bytes(c, 11 - (faces ? 5 : 0), 15 + (last ? 5 : 0) + (prim ? 7 : 0)));
-  if (c->f32()) launch_rk_next<float>(ew_grid(c), c->st, c->dbd, sp, c->dcc, last, prim, faces ? 0 : 1);
-  else launch_rk_next<double>(ew_grid(c), c->st, c->dbd, sp, c->dcc, last, prim, 1);
+  const bool forced = c->forced.ng + c->forced.ns > 0;
+  if (c->f32()) launch_rk_next<float>(ew_grid(c), c->st, c->dbd, sp, c->dcc, last, prim, faces ? 0 : 1, forced);
+  else launch_rk_next<double>(ew_grid(c), c->st, c->dbd, sp, c->dcc, last, prim, 1, forced);
   CK(cudaGetLastError());
   if (faces) {
     c->launches += 1;

@@ -2595,7 +2595,9 @@ __device__ __forceinline__ void rhs_of(const Work<R>& W, long long l, long long 
 // faces, the junction points); the FP32 fluxes of the next stage read the
 // primitives, and nothing else reads the interior state before the last stage
 // rewrites it.
-template <class R, bool STORE_Q = true>
+// FORCED false: no block of the context has such points (the test alone cost the
+// FP32 update 8 %).
+template <class R, bool STORE_Q, bool FORCED>
 __global__ void k_rk_next(const BlockDev* __restrict__ bd, const StageParams* __restrict__ sp,
                           const CaseConst* __restrict__ cc, int last, int prim) {
   FOR_POINTS(bd[blockIdx.y]) {
@@ -2607,7 +2609,7 @@ __global__ void k_rk_next(const BlockDev* __restrict__ bd, const StageParams* __
     // between two loads would hold the second behind the first's latency
     R dv[5];
     double qo[5];
-    if (B.forced && B.forced[l]) rhs_of<R, false>(W, l, n, dv);
+    if (FORCED && B.forced && B.forced[l]) rhs_of<R, false>(W, l, n, dv);
     else rhs_of<R, true>(W, l, n, dv);
 #pragma unroll
     for (int c = 0; c < 5; ++c) qo[c] = B.qo[l + c * n];
@@ -2917,9 +2919,10 @@ __global__ void k_rk_faces(const BlockDev* __restrict__ bd, const StageParams* _
 }
 template <class R>
 void launch_rk_next(dim3 g, cudaStream_t st, const BlockDev* bd, const StageParams* sp, const CaseConst* cc, int last,
-                    int prim, int store_q) {
-  if (store_q) k_rk_next<R, true><<<g, 256, 0, st>>>(bd, sp, cc, last, prim);
-  else k_rk_next<R, false><<<g, 256, 0, st>>>(bd, sp, cc, last, prim);
+                    int prim, int store_q, bool forced) {
+  if (forced) k_rk_next<R, true, true><<<g, 256, 0, st>>>(bd, sp, cc, last, prim);
+  else if (store_q) k_rk_next<R, true, false><<<g, 256, 0, st>>>(bd, sp, cc, last, prim);
+  else k_rk_next<R, false, false><<<g, 256, 0, st>>>(bd, sp, cc, last, prim);
 }
 template <class R>
 void launch_rk_faces(int grid, cudaStream_t st, const BlockDev* bd, const StageParams* sp, const int* tb,
