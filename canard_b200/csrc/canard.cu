@@ -1691,100 +1691,25 @@ void build_tables(canard_ctx* c) {
   }
 }
 
-// The averaging plans of all cases (AvgDev) and the points the walls reset,
-// whose primitives are redone with the averaged ones'.
-void build_average(canard_ctx* c, const AvgPlan& P, const AvgPlan& Lp0, const AvgPlan& Sf,
-                   const std::map<std::pair<int, long long>, int>& wall) {
-  typedef std::pair<int, long long> Pt;
-  // A line's mean over the point itself two or four times (an edge of a block
-  // that is periodic onto itself) is the point: x + x, then (2x + x) + x = 4x
-  // exactly, and the scaling is exact. Such targets fall away; eight copies (a
-  // corner) may round and stay.
-  AvgPlan Lk;
-  for (const AvgTarget& t : Lp0.targets) {
-    bool self = t.count == 1 || t.count == 2 || t.count == 4;
-    for (int j = 0; j < t.count; ++j)
-      self = self && Lp0.src_b[t.first + j] == t.b && Lp0.src_l[t.first + j] == t.l;
-    if (self) continue;
-    AvgTarget u = t;
-    u.first = (int)Lk.src_b.size();
-    Lk.src_b.insert(Lk.src_b.end(), Lp0.src_b.begin() + t.first, Lp0.src_b.begin() + t.first + t.count);
-    Lk.src_l.insert(Lk.src_l.end(), Lp0.src_l.begin() + t.first, Lp0.src_l.begin() + t.first + t.count);
-    Lk.targets.push_back(u);
-  }
-  const AvgPlan& Lp = Lk;
-  std::map<Pt, int> pt, ln;  // target index of a point
-  for (size_t k = 0; k < P.targets.size(); ++k) pt[{P.targets[k].b, (long long)P.targets[k].l}] = (int)k;
-  for (size_t k = 0; k < Lp.targets.size(); ++k) ln[{Lp.targets[k].b, (long long)Lp.targets[k].l}] = (int)k;
-  // a point as stored, after average_point, or after average_line; only points
-  // on a block edge can be targets of those two
-  auto ref = [&](int b, long long l, int stage) {
-    AvgRef r{b, -1, l};
-    const BlockGeom& g = c->blocks[b].g;
-    const int x = (int)(l % g.Xp), y = (int)(l / g.Xp % g.Y), z = (int)(l / ((long long)g.Xp * g.Y));
-    const int faces = (x == 0 || x == g.X - 1) + (y == 0 || y == g.Y - 1) + (z == 0 || z == g.Z - 1);
-    if (faces < 2) return r;
-    if (stage > 0) {
-      auto p = pt.find({b, l});
-      if (p != pt.end()) r.code = 2 * p->second;
-    }
-    if (stage > 1) {
-      auto q = ln.find({b, l});
-      if (q != ln.end()) r.code = 2 * q->second + 1;
-    }
-    return r;
-  };
-  auto refs = [&](const AvgPlan& p, int stage) {
-    std::vector<AvgRef> v;
-    v.reserve(p.src_b.size());
-    for (size_t e = 0; e < p.src_b.size(); ++e) v.push_back(ref(p.src_b[e], (long long)p.src_l[e], stage));
-    return v;
-  };
-  auto means = [&](const AvgPlan& p, int stage, AvgMeans& m) {
-    m.n = (int)p.targets.size();
+// the averaging tables of all cases and the points the walls reset
+void build_average(canard_ctx* c, const AvgTables& T) {
+  auto means = [&](const AvgTables::Means& t, AvgMeans& m) {
+    m.n = (int)t.first.size();
     if (m.n == 0) return;
-    std::vector<int> f, n;
-    for (const AvgTarget& t : p.targets) { f.push_back(t.first); n.push_back(t.count); }
-    m.first = dupload(f, c->st);
-    m.count = dupload(n, c->st);
-    m.src = dupload(refs(p, stage), c->st);
+    m.first = dupload(t.first, c->st);
+    m.count = dupload(t.count, c->st);
+    m.src = dupload(t.src, c->st);
     m.out = dalloc<double>((size_t)5 * m.n, c->st);
   };
   AvgDev& A = c->avg;
-  means(P, 0, A.pt);
-  means(Lp, 1, A.ln);
-  A.src = dupload(refs(Sf, 2), c->st);
-  // the points of all three plans in memory order, each with average_surface's partners
-  std::vector<std::pair<Pt, int>> all;
-  all.reserve(Sf.targets.size());
-  for (size_t k = 0; k < Sf.targets.size(); ++k) all.push_back({{Sf.targets[k].b, (long long)Sf.targets[k].l}, (int)k});
-  std::sort(all.begin(), all.end());
-  std::vector<std::pair<Pt, int>> more;  // on an edge or corner, but on no averaged face
-  auto known = [&](const Pt& p) {
-    auto it = std::lower_bound(all.begin(), all.end(), std::make_pair(p, -1));
-    return it != all.end() && it->first == p;
-  };
-  for (const auto* m : {&pt, &ln})
-    for (const auto& e : *m)
-      if (!known(e.first)) more.push_back({e.first, -1});
-  std::sort(more.begin(), more.end());
-  more.erase(std::unique(more.begin(), more.end()), more.end());
-  all.insert(all.end(), more.begin(), more.end());
-  std::vector<AvgRef> own;
-  std::vector<int> first, count;
-  for (const auto& e : all) {
-    own.push_back(ref(e.first.first, e.first.second, 2));
-    first.push_back(e.second < 0 ? 0 : Sf.targets[e.second].first);
-    count.push_back(e.second < 0 ? 0 : Sf.targets[e.second].count);
-  }
-  A.n = (int)own.size();
-  auto averaged = [&](const Pt& p) { return known(p) || pt.count(p) || ln.count(p); };
-  for (const auto& e : wall)
-    if (!averaged(e.first)) own.push_back({e.first.first, -1, e.first.second});
-  A.np = (int)own.size();
-  A.own = dupload(own, c->st);
-  A.first = dupload(first, c->st);
-  A.count = dupload(count, c->st);
+  means(T.pt, A.pt);
+  means(T.ln, A.ln);
+  A.n = (int)T.n;
+  A.np = (int)T.own.size();
+  A.own = dupload(T.own, c->st);
+  A.first = dupload(T.first, c->st);
+  A.count = dupload(T.count, c->st);
+  A.src = dupload(T.src, c->st);
   A.out = dalloc<double>((size_t)5 * A.n, c->st);
   CK(cudaStreamSynchronize(c->st));
 }
@@ -1956,31 +1881,14 @@ void build_gcbc_sponge_avg(canard_ctx* c) {
     };
     append(P, p1); append(Lp, l1); append(Sf, s1);
   }
-  // wall-face points with their resets in the reference's face order
-  std::map<std::pair<int, long long>, int> wall;
-  for (int b = 0; b < nb; ++b) {
-    const BlockGeom& g = c->blocks[b].g;
-    for (int nn = 1; nn <= 3; ++nn)
-      for (int ip = 0; ip <= 1; ++ip) {
-        const int np = g.nbc[nn - 1][ip];
-        if (np != BC_WALLI && np != BC_WALLV) continue;
-        const int pos = ip * g.ijk[0][nn - 1];
-        for (int k = 0; k <= g.ijk[2][nn - 1]; ++k)
-          for (int j = 0; j <= g.ijk[1][nn - 1]; ++j) {
-            int x, y, z;
-            g.line_xyz(nn, pos, j, k, x, y, z);
-            int& kinds = wall[{b, (long long)g.dev(x, y, z)}];
-            int s = 0;
-            while ((kinds >> (2 * s)) & 3) ++s;
-            kinds |= (np == BC_WALLI ? 1 : 2) << (2 * s);
-          }
-      }
-  }
+  std::vector<const BlockGeom*> geoms;
+  for (const BlockState& B : c->blocks) geoms.push_back(&B.g);
+  const std::vector<WallPoint> wall = wall_points(geoms);
   c->wall_n = (int)wall.size();
   if (c->wall_n) {
     std::vector<int> wb, wk;
     std::vector<long long> wl;
-    for (const auto& e : wall) { wb.push_back(e.first.first); wl.push_back(e.first.second); wk.push_back(e.second); }
+    for (const WallPoint& e : wall) { wb.push_back(e.b); wl.push_back(e.l); wk.push_back(e.kinds); }
     c->wall_tb = dupload(wb, c->st);
     c->wall_tl = dupload(wl, c->st);
     c->wall_tk = dupload(wk, c->st);
@@ -2005,7 +1913,7 @@ void build_gcbc_sponge_avg(canard_ctx* c) {
       c->face_tl = dupload(fl, c->st);
     }
   }
-  build_average(c, P, Lp, Sf, wall);
+  build_average(c, average_tables(geoms, P, Lp, Sf, wall));
 }
 
 // t_grid%grid_metrics on the device (src/mo_grid.f90:52-189)

@@ -643,6 +643,115 @@ std::string surface_plan(const std::vector<BlockGeom>& B, const std::vector<Face
   return "";
 }
 
+std::vector<WallPoint> wall_points(const std::vector<const BlockGeom*>& B) {
+  std::map<std::pair<int, int64_t>, int> wall;
+  for (int b = 0; b < (int)B.size(); ++b) {
+    const BlockGeom& g = *B[b];
+    for (int nn = 1; nn <= 3; ++nn)
+      for (int ip = 0; ip <= 1; ++ip) {
+        const int np = g.nbc[nn - 1][ip];
+        if (np != BC_WALLI && np != BC_WALLV) continue;
+        const int pos = ip * g.ijk[0][nn - 1];
+        for (int k = 0; k <= g.ijk[2][nn - 1]; ++k)
+          for (int j = 0; j <= g.ijk[1][nn - 1]; ++j) {
+            int x, y, z;
+            g.line_xyz(nn, pos, j, k, x, y, z);
+            int& kinds = wall[{b, g.dev(x, y, z)}];
+            int s = 0;
+            while ((kinds >> (2 * s)) & 3) ++s;
+            kinds |= (np == BC_WALLI ? 1 : 2) << (2 * s);
+          }
+      }
+  }
+  std::vector<WallPoint> v;
+  for (const auto& e : wall) v.push_back({e.first.first, e.first.second, e.second});
+  return v;
+}
+
+AvgTables average_tables(const std::vector<const BlockGeom*>& B, const AvgPlan& P, const AvgPlan& Lp0,
+                         const AvgPlan& Sf, const std::vector<WallPoint>& wall) {
+  typedef std::pair<int, int64_t> Pt;
+  // A line's mean over the point itself two or four times (an edge of a block
+  // that is periodic onto itself) is the point: x + x, then (2x + x) + x = 4x
+  // exactly, and the scaling is exact. Such targets fall away; eight copies (a
+  // corner) may round and stay.
+  AvgPlan Lp;
+  for (const AvgTarget& t : Lp0.targets) {
+    bool self = t.count == 1 || t.count == 2 || t.count == 4;
+    for (int j = 0; j < t.count; ++j)
+      self = self && Lp0.src_b[t.first + j] == t.b && Lp0.src_l[t.first + j] == t.l;
+    if (self) continue;
+    AvgTarget u = t;
+    u.first = (int)Lp.src_b.size();
+    Lp.src_b.insert(Lp.src_b.end(), Lp0.src_b.begin() + t.first, Lp0.src_b.begin() + t.first + t.count);
+    Lp.src_l.insert(Lp.src_l.end(), Lp0.src_l.begin() + t.first, Lp0.src_l.begin() + t.first + t.count);
+    Lp.targets.push_back(u);
+  }
+  std::map<Pt, int> pt, ln;  // target index of a point
+  for (size_t k = 0; k < P.targets.size(); ++k) pt[{P.targets[k].b, P.targets[k].l}] = (int)k;
+  for (size_t k = 0; k < Lp.targets.size(); ++k) ln[{Lp.targets[k].b, Lp.targets[k].l}] = (int)k;
+  // a point as stored, after average_point, or after average_line; only points
+  // on a block edge can be targets of those two
+  auto ref = [&](int b, int64_t l, int stage) {
+    AvgRef r{b, -1, l};
+    const BlockGeom& g = *B[b];
+    const int x = (int)(l % g.Xp), y = (int)(l / g.Xp % g.Y), z = (int)(l / ((int64_t)g.Xp * g.Y));
+    const int faces = (x == 0 || x == g.X - 1) + (y == 0 || y == g.Y - 1) + (z == 0 || z == g.Z - 1);
+    if (faces < 2) return r;
+    if (stage > 0) {
+      auto p = pt.find({b, l});
+      if (p != pt.end()) r.code = 2 * p->second;
+    }
+    if (stage > 1) {
+      auto q = ln.find({b, l});
+      if (q != ln.end()) r.code = 2 * q->second + 1;
+    }
+    return r;
+  };
+  auto refs = [&](const AvgPlan& p, int stage) {
+    std::vector<AvgRef> v;
+    v.reserve(p.src_b.size());
+    for (size_t e = 0; e < p.src_b.size(); ++e) v.push_back(ref(p.src_b[e], p.src_l[e], stage));
+    return v;
+  };
+  auto means = [&](const AvgPlan& p, int stage, AvgTables::Means& m) {
+    for (const AvgTarget& t : p.targets) { m.first.push_back(t.first); m.count.push_back(t.count); }
+    m.src = refs(p, stage);
+  };
+  AvgTables T;
+  means(P, 0, T.pt);
+  means(Lp, 1, T.ln);
+  T.src = refs(Sf, 2);
+  // the points of all three plans in memory order, each with average_surface's partners
+  std::vector<std::pair<Pt, int>> all;
+  all.reserve(Sf.targets.size());
+  for (size_t k = 0; k < Sf.targets.size(); ++k) all.push_back({{Sf.targets[k].b, Sf.targets[k].l}, (int)k});
+  std::sort(all.begin(), all.end());
+  std::vector<std::pair<Pt, int>> more;  // on an edge or corner, but on no averaged face
+  const size_t nface = all.size();       // sorted; what is appended behind is a run of its own
+  auto known = [&](const Pt& p) {        // on an averaged face
+    const auto end = all.begin() + nface;
+    auto it = std::lower_bound(all.begin(), end, std::make_pair(p, -1));
+    return it != end && it->first == p;
+  };
+  for (const auto* m : {&pt, &ln})
+    for (const auto& e : *m)
+      if (!known(e.first)) more.push_back({e.first, -1});
+  std::sort(more.begin(), more.end());
+  more.erase(std::unique(more.begin(), more.end()), more.end());
+  all.insert(all.end(), more.begin(), more.end());
+  for (const auto& e : all) {
+    T.own.push_back(ref(e.first.first, e.first.second, 2));
+    T.first.push_back(e.second < 0 ? 0 : Sf.targets[e.second].first);
+    T.count.push_back(e.second < 0 ? 0 : Sf.targets[e.second].count);
+  }
+  T.n = T.own.size();
+  auto averaged = [&](const Pt& p) { return known(p) || pt.count(p) || ln.count(p); };
+  for (const WallPoint& e : wall)
+    if (!averaged({e.b, e.l})) T.own.push_back({e.b, -1, e.l});
+  return T;
+}
+
 void gcbc_tables(const BlockGeom& g, const double* yaco, std::vector<GcbcFace>& faces,
                  std::vector<int64_t>& pts, std::vector<double>& w) {
   // taper weights of the 4 inward points: sbci = -cbca^-1 rbci, times a cosine
@@ -822,6 +931,74 @@ extern "C" int canard_average_host(int32_t nranks, const canard_block_desc* rank
         for (int y = 0; y < g.Y; ++y)
           for (int x = 0; x < g.X; ++x)
             qa[r][(size_t)c * g.X * g.Y * g.Z + g.ref_index(x, y, z)] = q[r][(size_t)c * g.npad + g.dev(x, y, z)];
+  }
+  return CANARD_OK;
+}
+
+
+// The same through the tables the device reads (average_tables; k_avg_mean,
+// k_avg_faces and k_average_store in this order), with the points that the last
+// of these launches writes, one thread each: own, 2 values per point (rank, point
+// l in the reference layout), the averaged ones first (*navg of them), then those
+// that only walls reset. Not part of the public header: the check of the tables
+// without a GPU.
+extern "C" int canard_average_tables_host(int32_t nranks, const canard_block_desc* ranks, int32_t nblocks,
+                                          const int32_t* nbpc, const int32_t* mbcd, const int32_t* sub,
+                                          double* const* qa, int64_t* own, int64_t cap, int64_t* n, int64_t* navg) {
+  using namespace canard;
+  if (nranks < 1 || !ranks || !qa || !n || !navg || cap < 0 || (cap > 0 && !own)) return CANARD_ERR_ARG;
+  for (int r = 0; r < nranks; ++r)
+    if (!qa[r]) return CANARD_ERR_ARG;
+  std::vector<BlockGeom> B;
+  std::vector<FaceLink> links;
+  AvgPlan P, L, S;
+  if (int rc = case_plans(nranks, ranks, nblocks, nbpc, mbcd, sub, B, links, P, L, S)) return rc;
+  std::vector<const BlockGeom*> geoms;
+  for (const BlockGeom& g : B) geoms.push_back(&g);
+  const AvgTables T = average_tables(geoms, P, L, S, wall_points(geoms));
+  *n = 2 * (int64_t)T.own.size();
+  *navg = (int64_t)T.n;
+  if (cap == 0) return CANARD_OK;
+  if (cap < *n) return CANARD_ERR_ARG;
+  auto at = [&](const AvgRef& r) {  // index in the reference's layout
+    const BlockGeom& g = B[r.b];
+    return g.ref_index((int)(r.l % g.Xp), (int)(r.l / g.Xp % g.Y), (int)(r.l / ((int64_t)g.Xp * g.Y)));
+  };
+  auto pts = [&](const AvgRef& r) { return (size_t)B[r.b].X * B[r.b].Y * B[r.b].Z; };
+  std::vector<double> pt(5 * T.pt.first.size()), ln(5 * T.ln.first.size()), out(5 * T.n);
+  auto value = [&](const AvgRef& r, double q[5]) {
+    for (int c = 0; c < 5; ++c)
+      q[c] = r.code < 0 ? qa[r.b][c * pts(r) + at(r)] : ((r.code & 1) ? ln : pt)[5 * (size_t)(r.code >> 1) + c];
+  };
+  auto means = [&](const AvgTables::Means& m, std::vector<double>& o) {
+    for (size_t t = 0; t < m.first.size(); ++t) {
+      double q[5], v[5];
+      for (int j = 0; j < m.count[t]; ++j) {
+        value(m.src[m.first[t] + j], v);
+        for (int c = 0; c < 5; ++c) q[c] = j == 0 ? v[c] : q[c] + v[c];
+      }
+      for (int c = 0; c < 5; ++c) o[5 * t + c] = (1.0 / (double)m.count[t]) * q[c];
+    }
+  };
+  means(T.pt, pt);
+  means(T.ln, ln);
+  for (size_t t = 0; t < T.n; ++t) {
+    double q[5], v[5], r1 = 1.0;
+    value(T.own[t], q);
+    for (int j = 0; j < T.count[t]; ++j) {
+      value(T.src[T.first[t] + j], v);
+      r1 = r1 + 1.0;
+      const double r2 = 1.0 / r1;
+      for (int c = 0; c < 5; ++c) q[c] = r2 * ((r1 - 1.0) * q[c] + v[c]) + 0.0 * q[c];
+    }
+    for (int c = 0; c < 5; ++c) out[5 * t + c] = q[c];
+  }
+  for (size_t t = 0; t < T.own.size(); ++t) {
+    const AvgRef& r = T.own[t];
+    if (t < T.n)
+      for (int c = 0; c < 5; ++c) qa[r.b][c * pts(r) + at(r)] = out[5 * t + c];
+    own[2 * t] = r.b;
+    own[2 * t + 1] = (int64_t)at(r);
   }
   return CANARD_OK;
 }

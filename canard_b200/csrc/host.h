@@ -95,6 +95,33 @@ std::string junction_plans(const std::vector<BlockGeom>& ranks, const Decomp& d,
 std::string surface_plan(const std::vector<BlockGeom>& blocks, const std::vector<FaceLink>& links,
                          AvgPlan& surf);
 
+// Points on wall faces with their resets (1 inviscid, 2 viscous, two bits each)
+// in the reference's face order, in memory order.
+struct WallPoint { int b; int64_t l; int kinds; };
+std::vector<WallPoint> wall_points(const std::vector<const BlockGeom*>& blocks);
+
+// A point of the state as one of the averaging routines reads it.
+struct AvgRef {
+  int b, code;  // code -1: as stored; 2k: average_point's result k; 2k+1: average_line's result k
+  int64_t l;
+};
+// The averaging plans as the device applies them (AvgDev): the means of points
+// and lines, then the running averages of all averaged points, own[0, n), and
+// behind those the points that only walls reset. Every point stands in own once:
+// one thread each stores its state and its primitives.
+struct AvgTables {
+  struct Means {
+    std::vector<int> first, count;
+    std::vector<AvgRef> src;
+  } pt, ln;
+  std::vector<AvgRef> own;
+  size_t n = 0;                   // averaged points
+  std::vector<int> first, count;  // [n] average_surface's partners in src
+  std::vector<AvgRef> src;
+};
+AvgTables average_tables(const std::vector<const BlockGeom*>& blocks, const AvgPlan& points, const AvgPlan& lines,
+                         const AvgPlan& surf, const std::vector<WallPoint>& wall);
+
 // GCBC weights (gcbc_init, src/mo_gcbc.f90:40-131): for each GCBC face of the
 // block in reference order, per line 5 (device point, weight) entries.
 struct GcbcFace { int nn, side, bc; int64_t first; };  // first entry = line 0, offset 0

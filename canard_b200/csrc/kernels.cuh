@@ -15,6 +15,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "host.h"
+
 namespace canard {
 
 constexpr int kLanes = 32;            // lines per tile (one warp, one line per lane)
@@ -2162,10 +2164,6 @@ __global__ void k_prim(const BlockDev* __restrict__ bd, const CaseConst* __restr
 // launches a stage of 2-16 us each whatever the size; one launch that evaluated
 // edges on the spot took longer than all of them (dependent loads of the few
 // corner threads: 20 steps of TGV 64 15.6 -> 16.4 ms).
-struct AvgRef {   // a point of the state as one of the routines reads it
-  int b, code;    // code -1: as stored; 2k: average_point's result k; 2k+1: average_line's result k
-  long long l;
-};
 struct AvgMeans {  // average_point's or average_line's targets: means over src[first, first + count)
   int n = 0;
   const int *first = nullptr, *count = nullptr;
