@@ -11,9 +11,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
-#include <atomic>
 #include <mutex>
-#include <system_error>
 #include <thread>
 #include <stdexcept>
 #include <string>
@@ -411,8 +409,6 @@ struct canard_ctx {
   cudaStream_t s_in = nullptr, s_out = nullptr;
   // copies of outputs into pageable host memory (copy_out): per worker thread a
   // pinned chunk and a stream
-  static constexpr int kCopyWorkers = 8;
-  static constexpr size_t kCopyChunk = 2u << 20;
   void* cp_pin[kCopyWorkers] = {};
   cudaStream_t cp_st[kCopyWorkers] = {};
   cudaEvent_t cp_ready = nullptr;
@@ -2018,57 +2014,50 @@ void d2h_field(canard_ctx* c, const BlockState& B, double* dst, const double* sr
   CK(cudaMemcpyAsync(dst, c->stage, n * sizeof(double), cudaMemcpyDeviceToHost, c->st));
 }
 
-// Copies a large output (written by work on c->st) into the caller's memory and
+// Copies an output (written by work on c->st) into the caller's memory and
 // returns when it is there. A new pageable array costs a page fault per 4 KB
 // besides the copy, all on the thread that asks the driver for it (340 MB: 70
-// ms), so a few threads each move chunks through a pinned buffer of their own:
-// transfers, copies and faults of different chunks overlap. Small copies and
-// pinned arrays go straight.
+// ms), so a few threads share large ones (see CopySource): transfers, copies and
+// faults of different chunks overlap. Pinned arrays go straight.
 void copy_out(canard_ctx* c, void* dst, const void* src, size_t bytes) {
-  constexpr size_t chunk = canard_ctx::kCopyChunk;
-  const size_t chunks = (bytes + chunk - 1) / chunk;
+  struct Device : CopySource {
+    canard_ctx* c;
+    const char* src;
+    size_t bytes;
+    int dev = 0;
+    bool open(int w) override {
+      cudaError_t e = cudaSuccess;
+      if (!c->cp_ready) e = cudaEventCreateWithFlags(&c->cp_ready, cudaEventDisableTiming);
+      if (e == cudaSuccess && !c->cp_pin[w]) e = cudaMallocHost(&c->cp_pin[w], kCopyChunk);
+      if (e == cudaSuccess && !c->cp_st[w]) e = cudaStreamCreateWithFlags(&c->cp_st[w], cudaStreamNonBlocking);
+      if (e == cudaSuccess) e = cudaEventRecord(c->cp_ready, c->st);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(c->cp_st[w], c->cp_ready, 0);
+      if (e != cudaSuccess) cudaGetLastError();
+      return e == cudaSuccess;
+    }
+    int fetch(int w, size_t off, size_t n, const void** p) override {
+      *p = c->cp_pin[w];
+      cudaError_t e = cudaSetDevice(dev);
+      if (e == cudaSuccess) e = cudaMemcpyAsync(c->cp_pin[w], src + off, n, cudaMemcpyDeviceToHost, c->cp_st[w]);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(c->cp_st[w]);
+      return (int)e;
+    }
+    int straight(void* d) override {
+      const cudaError_t e = cudaMemcpyAsync(d, src, bytes, cudaMemcpyDeviceToHost, c->st);
+      return (int)(e == cudaSuccess ? cudaStreamSynchronize(c->st) : e);
+    }
+  } s;
+  s.c = c;
+  s.src = static_cast<const char*>(src);
+  s.bytes = bytes;
+  CK(cudaGetDevice(&s.dev));
   cudaPointerAttributes at{};
   if (cudaPointerGetAttributes(&at, dst) != cudaSuccess) {
     cudaGetLastError();
     at.type = cudaMemoryTypeUnregistered;
   }
-  const int workers = (int)std::min<size_t>(std::min<size_t>(canard_ctx::kCopyWorkers, chunks),
-                                            std::max(1u, std::thread::hardware_concurrency()));
-  if (workers < 2 || at.type != cudaMemoryTypeUnregistered) {
-    CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    return;
-  }
-  int dev = 0;
-  CK(cudaGetDevice(&dev));
-  if (!c->cp_ready) CK(cudaEventCreateWithFlags(&c->cp_ready, cudaEventDisableTiming));
-  for (int w = 0; w < workers; ++w) {
-    if (!c->cp_pin[w]) CK(cudaMallocHost(&c->cp_pin[w], chunk));
-    if (!c->cp_st[w]) CK(cudaStreamCreateWithFlags(&c->cp_st[w], cudaStreamNonBlocking));
-  }
-  CK(cudaEventRecord(c->cp_ready, c->st));
-  std::atomic<size_t> next{0};
-  std::atomic<int> failed{0};
-  auto work = [&](int w) {
-    cudaError_t e = cudaSetDevice(dev);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(c->cp_st[w], c->cp_ready, 0);
-    for (size_t k; e == cudaSuccess && (k = next.fetch_add(1)) < chunks;) {
-      const size_t off = k * chunk, n = std::min(chunk, bytes - off);
-      e = cudaMemcpyAsync(c->cp_pin[w], static_cast<const char*>(src) + off, n, cudaMemcpyDeviceToHost, c->cp_st[w]);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(c->cp_st[w]);
-      if (e == cudaSuccess) std::memcpy(static_cast<char*>(dst) + off, c->cp_pin[w], n);
-    }
-    if (e != cudaSuccess) failed.store((int)e);
-  };
-  std::vector<std::thread> pool;
-  try {
-    for (int w = 1; w < workers; ++w) pool.emplace_back(work, w);
-  } catch (const std::system_error&) {
-    // fewer threads than asked for: the ones there take the chunks
-  }
-  work(0);
-  for (auto& t : pool) t.join();
-  CK(static_cast<cudaError_t>(failed.load()));
+  const int workers = at.type != cudaMemoryTypeUnregistered ? 1 : copy_workers(bytes, std::thread::hardware_concurrency());
+  CK(static_cast<cudaError_t>(copy_out(s, dst, bytes, workers)));
 }
 
 int block_index(const canard_ctx* c, int icase, int iblock) {

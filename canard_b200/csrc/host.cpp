@@ -4,11 +4,13 @@
 #include "host.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <deque>
 #include <map>
 #include <stdexcept>
+#include <thread>
 #include <tuple>
 
 namespace canard {
@@ -830,6 +832,39 @@ void sponge_list(const BlockGeom& g, const canard_case_desc& c, const double* xy
   }
 }
 
+int copy_workers(size_t bytes, unsigned cores) {
+  const size_t most = std::min<size_t>(kCopyWorkers, std::max(1u, cores));
+  return (int)std::max<size_t>(1, std::min(most, (bytes + kCopyChunk - 1) / kCopyChunk));
+}
+
+int copy_out(CopySource& s, void* dst, size_t bytes, int workers) {
+  int n = 0;
+  while (workers > 1 && n < workers && s.open(n)) ++n;
+  if (n < 2) return s.straight(dst);
+  const size_t chunks = (bytes + kCopyChunk - 1) / kCopyChunk;
+  std::atomic<size_t> next{0};
+  std::atomic<int> failed{0};
+  auto work = [&](int w) {
+    for (size_t k; failed.load() == 0 && (k = next.fetch_add(1)) < chunks;) {
+      const size_t off = k * kCopyChunk, len = std::min(kCopyChunk, bytes - off);
+      const void* p = nullptr;
+      const int e = s.fetch(w, off, len, &p);
+      if (e != 0) failed.store(e);
+      else std::memcpy(static_cast<char*>(dst) + off, p, len);
+    }
+  };
+  std::vector<std::thread> pool;
+  pool.reserve((size_t)n);
+  try {
+    for (int w = 1; w < n; ++w) pool.emplace_back(work, w);
+  } catch (const std::exception&) {
+    // fewer threads than asked for: the ones there take the chunks
+  }
+  work(0);
+  for (auto& t : pool) t.join();
+  return failed.load();
+}
+
 }  // namespace canard
 
 namespace {
@@ -1001,6 +1036,45 @@ extern "C" int canard_average_tables_host(int32_t nranks, const canard_block_des
     own[2 * t + 1] = (int64_t)at(r);
   }
   return CANARD_OK;
+}
+
+
+// copy_out with a stand-in for the device: open(w) fails from worker `opens` on,
+// fetch fails with code 7 at chunk `bad` (-1: none). *used receives the workers
+// that were opened, or 0 if the copy went straight. Not part of the public
+// header: the check of the threads without a GPU.
+extern "C" int canard_copy_out_host(const char* src, char* dst, int64_t bytes, int32_t cores,
+                                    int32_t opens, int64_t bad, int32_t* used) {
+  using namespace canard;
+  struct Host : CopySource {
+    const char* src;
+    size_t bytes;
+    int opens, opened = 0, bad;
+    bool went_straight = false;
+    std::vector<std::vector<char>> buf;
+    bool open(int w) override {
+      if (w >= opens) return false;
+      ++opened;
+      buf.emplace_back(kCopyChunk);
+      return true;
+    }
+    int fetch(int w, size_t off, size_t n, const void** p) override {
+      if (bad >= 0 && off / kCopyChunk == (size_t)bad) return 7;
+      std::memcpy(buf[w].data(), src + off, n);
+      *p = buf[w].data();
+      return 0;
+    }
+    int straight(void* d) override {
+      went_straight = true;
+      std::memcpy(d, src, bytes);
+      return 0;
+    }
+  } h;
+  if (!src || !dst || bytes < 0 || !used) return CANARD_ERR_ARG;
+  h.src = src; h.bytes = (size_t)bytes; h.opens = opens; h.bad = (int)bad;
+  const int rc = copy_out(h, dst, (size_t)bytes, copy_workers((size_t)bytes, (unsigned)std::max(0, cores)));
+  *used = h.went_straight ? 0 : h.opened;
+  return rc;
 }
 
 

@@ -133,4 +133,21 @@ void sponge_list(const BlockGeom& g, const canard_case_desc& c, const double* xy
                  const double* yaco_ref, std::vector<int64_t>& pts, std::vector<double>& asz,
                  std::vector<double>& bsz);
 
+// Copies of large outputs from the device into the caller's pageable memory, by
+// a few threads that each move chunks through a pinned buffer of their own.
+// Workers of an output of `bytes` (1: straight).
+constexpr int kCopyWorkers = 8;
+constexpr size_t kCopyChunk = 2u << 20;
+int copy_workers(size_t bytes, unsigned cores);
+struct CopySource {
+  virtual ~CopySource() = default;
+  virtual bool open(int w) = 0;  // worker w's buffer and stream; false: cannot be had
+  // bytes [off, off + n) of the output where worker w can read them; an error code or 0
+  virtual int fetch(int w, size_t off, size_t n, const void** p) = 0;
+  virtual int straight(void* dst) = 0;  // the whole output by one copy; an error code or 0
+};
+// Returns when the output is in dst. The caller's memory needs no worker: with
+// fewer than two that can be opened the output goes straight.
+int copy_out(CopySource& s, void* dst, size_t bytes, int workers);
+
 }  // namespace canard
