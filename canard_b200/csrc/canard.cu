@@ -408,10 +408,11 @@ struct canard_ctx {
   size_t hs_n = 0;
   cudaStream_t s_in = nullptr, s_out = nullptr;
   // copies of outputs into pageable host memory (copy_out): per worker thread a
-  // pinned chunk and a stream
+  // pinned chunk and a stream; bytes copied so far
   void* cp_pin[kCopyWorkers] = {};
   cudaStream_t cp_st[kCopyWorkers] = {};
   cudaEvent_t cp_ready = nullptr;
+  size_t cp_before = 0;
   size_t stage_n = 0;
   int* derr = nullptr;
   bool setup_done = false;
@@ -2056,7 +2057,11 @@ void copy_out(canard_ctx* c, void* dst, const void* src, size_t bytes) {
     cudaGetLastError();
     at.type = cudaMemoryTypeUnregistered;
   }
-  const int workers = at.type != cudaMemoryTypeUnregistered ? 1 : copy_workers(bytes, std::thread::hardware_concurrency());
+  int workers = 1;
+  if (at.type == cudaMemoryTypeUnregistered) {
+    workers = copy_workers(bytes, c->cp_before, std::thread::hardware_concurrency());
+    c->cp_before += bytes;
+  }
   CK(static_cast<cudaError_t>(copy_out(s, dst, bytes, workers)));
 }
 

@@ -832,7 +832,8 @@ void sponge_list(const BlockGeom& g, const canard_case_desc& c, const double* xy
   }
 }
 
-int copy_workers(size_t bytes, unsigned cores) {
+int copy_workers(size_t bytes, size_t before, unsigned cores) {
+  if (bytes + before < kCopyStraight) return 1;
   const size_t most = std::min<size_t>(kCopyWorkers, std::max(1u, cores));
   return (int)std::max<size_t>(1, std::min(most, (bytes + kCopyChunk - 1) / kCopyChunk));
 }
@@ -1043,7 +1044,7 @@ extern "C" int canard_average_tables_host(int32_t nranks, const canard_block_des
 // fetch fails with code 7 at chunk `bad` (-1: none). *used receives the workers
 // that were opened, or 0 if the copy went straight. Not part of the public
 // header: the check of the threads without a GPU.
-extern "C" int canard_copy_out_host(const char* src, char* dst, int64_t bytes, int32_t cores,
+extern "C" int canard_copy_out_host(const char* src, char* dst, int64_t bytes, int64_t before, int32_t cores,
                                     int32_t opens, int64_t bad, int32_t* used) {
   using namespace canard;
   struct Host : CopySource {
@@ -1070,9 +1071,9 @@ extern "C" int canard_copy_out_host(const char* src, char* dst, int64_t bytes, i
       return 0;
     }
   } h;
-  if (!src || !dst || bytes < 0 || !used) return CANARD_ERR_ARG;
+  if (!src || !dst || bytes < 0 || before < 0 || !used) return CANARD_ERR_ARG;
   h.src = src; h.bytes = (size_t)bytes; h.opens = opens; h.bad = (int)bad;
-  const int rc = copy_out(h, dst, (size_t)bytes, copy_workers((size_t)bytes, (unsigned)std::max(0, cores)));
+  const int rc = copy_out(h, dst, (size_t)bytes, copy_workers((size_t)bytes, (size_t)before, (unsigned)std::max(0, cores)));
   *used = h.went_straight ? 0 : h.opened;
   return rc;
 }

@@ -135,10 +135,16 @@ void sponge_list(const BlockGeom& g, const canard_case_desc& c, const double* xy
 
 // Copies of large outputs from the device into the caller's pageable memory, by
 // a few threads that each move chunks through a pinned buffer of their own.
-// Workers of an output of `bytes` (1: straight).
+// Workers of an output of `bytes` (1: straight) after `before` bytes of outputs.
+// A worker costs about 1.7 ms to set up (2 MiB pinned, a stream), and only new
+// pages make threads pay: 41 MiB 10.4 ms straight and 2.2 by 8 threads, 324 MiB
+// 73 and 13, but 20 MiB in used pages 1.3 and 1.2. So the first 64 MiB of a
+// context's outputs go straight: with threads from 2 MiB on a first output of 5
+// MiB took 5-9 ms, of 20 MiB 16-50, of 41 MiB 16; straight 1.0, 3-4 and 10.4 (80
+// MiB: 18 and 19). Chunks of 1 MiB cost half the set-up, but 324 MiB took 16.9 ms.
 constexpr int kCopyWorkers = 8;
-constexpr size_t kCopyChunk = 2u << 20;
-int copy_workers(size_t bytes, unsigned cores);
+constexpr size_t kCopyChunk = 2u << 20, kCopyStraight = 64u << 20;
+int copy_workers(size_t bytes, size_t before, unsigned cores);
 struct CopySource {
   virtual ~CopySource() = default;
   virtual bool open(int w) = 0;  // worker w's buffer and stream; false: cannot be had
