@@ -1565,11 +1565,23 @@ int longest_line(const canard_ctx* c, int dir) {
   return L;
 }
 
+// Tiles of the context's longest lines (derivative nt 0, filter 1) that an SM's
+// shared memory holds at once; 0: not even one fits a CTA.
+int tiles_per_sm(const canard_ctx* c, int nt, int dir, int kind) {
+  const BlockState* B = &c->blocks[0];
+  for (const auto& b : c->blocks)
+    if (b.g.ijk[0][dir] > B->g.ijk[0][dir]) B = &b;
+  LineTask t;
+  fill_line_task(c, *B, dir, nt, nullptr, nullptr, 1, false, t, kind);
+  const size_t bytes = line_smem(dir, t, kind);
+  return bytes > (size_t)kLineSmemMax ? 0 : (int)((228 * 1024) / (bytes + 1024));  // 1 KiB reserved per CTA
+}
+
 // Defaults without autotuning, five fields, ms per launch on a B200. The
 // one-lane sweeps keep whole lines of 32 in a CTA, so their rate falls where
-// fewer than four tiles fit an SM (FP64: lines of more than about 200 points);
-// the two-ended solve halves the dependent chain there at the price of more
-// start-up per tile.
+// fewer than four tiles fit an SM (FP64: lines of more than about 200 points,
+// FP32 420); the two-ended solve halves the dependent chain there at the price
+// of more start-up per tile, the split solve also the tile.
 // Fast mode, derivative, one-lane against two-ended: 65 points (zeta of
 // 193 x 129 x 65) 0.040 / 0.057, 129 points 0.039 / 0.048, 193 points 0.047 /
 // 0.054, 257 points 0.294-0.319 / 0.300-0.306, 385 points 0.295 / 0.274.
@@ -1577,15 +1589,28 @@ int longest_line(const canard_ctx* c, int dir) {
 // points 0.049 / 0.047, 257 points 0.39-0.49 / 0.34-0.42.
 // Mixed precision, derivative, one-lane against split: 65 points 0.027 /
 // 0.046, 129 points 0.025 / 0.033, 257 points 0.139-0.147 / 0.167-0.189, 385
-// points 0.125 / 0.135. Its filter runs in FP64 like the fast mode's where the
-// two-ended FP32 elimination is the slower one (257 points 0.34-0.43 / 0.36-0.50).
+// points 0.125 / 0.135; 5.6 M points a field: xi 433 points (four tiles) 0.067 /
+// 0.076, 449 (three) 0.077 / 0.068, 513 0.085 / 0.070, 897 0.161 / 0.092, 1537
+// 0.150 / 0.095; eta 417 (four) 0.067 / 0.074, 433 (three) 0.089 / 0.070, 1025
+// 0.126 / 0.078, 1785 0.158 / 0.109, 1801 (one tile of either) 0.160 / 0.176.
+// The mixed filter runs in FP64 like the fast mode's where the two-ended FP32
+// elimination is the slower one (257 points 0.34-0.43 / 0.36-0.50).
+// Without a two-ended tile (lines too long for it, or a block with lines under
+// 32 points), FP64, one-lane against split, 5.6 M points: derivative 257 points
+// (three tiles) 0.119 / 0.129 along xi, 0.109 / 0.117 along eta, 321 (two) 0.147 /
+// 0.133 and 0.124 / 0.110, 897 0.231 / 0.169; filter along xi 385 (two) 0.178 /
+// 0.207, 513 (one) 0.310 / 0.214, 897 0.298 / 0.225, along eta 321 0.176 / 0.222,
+// 641 0.285 / 0.333, 881 0.227 / 0.250.
 int default_kind(const canard_ctx* c, int grp, int dir) {
   if (!c->fast() && !c->f32()) return LK_F64;
-  const int L = longest_line(c, dir);
-  auto fits = [&](int kind) { return tile_smem_for(dir, L, kind) <= (size_t)kLineSmemMax; };
-  if (c->f32() && grp != 0) return fits(LK_F32_1L) ? LK_F32_1L : LK_F32;
-  if (twist_ok(c, dir, LK_F64_TWIST) && L > (grp == 0 ? 160 : 200)) return LK_F64_TWIST;
-  return fits(LK_F64_1L) ? LK_F64_1L : LK_F64_SPLIT;
+  const int nt = grp == 0 ? 1 : 0;
+  if (c->f32() && grp != 0) {
+    const int one = tiles_per_sm(c, nt, dir, LK_F32_1L);
+    return one >= 4 || (one >= 1 && tiles_per_sm(c, nt, dir, LK_F32) < 2) ? LK_F32_1L : LK_F32;
+  }
+  if (twist_ok(c, dir, LK_F64_TWIST) && longest_line(c, dir) > (grp == 0 ? 160 : 200)) return LK_F64_TWIST;
+  const int least = grp != 0 ? 3 : dir == 0 ? 2 : 1;
+  return tiles_per_sm(c, nt, dir, LK_F64_1L) >= least ? LK_F64_1L : LK_F64_SPLIT;
 }
 
 int group_kind(const canard_ctx* c, int grp, int dir) {
