@@ -2366,6 +2366,41 @@ void create(canard_ctx* c, const canard_case_desc* cases, int ncases, const cana
   CK(cudaStreamSynchronize(c->st));
 }
 
+// the line kinds the autotuner tries for a group and direction, each once, the
+// default first; all of them kinds that canard_set_line_kind takes there
+std::vector<int> tune_kinds(const canard_ctx* c, int grp, int dir) {
+  std::vector<int> kinds{default_kind(c, grp, dir)};
+  auto add = [&](std::initializer_list<int> ks) { kinds.insert(kinds.end(), ks); };
+  if (!c->f32()) {
+    if (c->fast()) {  // the one-lane and split FP64 sweeps compete in the fast mode
+      add({LK_F64, LK_F64_1L, LK_F64_SPLIT});
+      if (grp != 0 && quad_ok(c, dir, LK_F64_QUAD)) add({LK_F64_QUAD});
+      if (twist_ok(c, dir, LK_F64_TWIST)) add({LK_F64_TWIST});
+    }
+    if (tm_ok(c, dir)) add({LK_F64_TM});
+  } else if (grp != 0) {  // FP32 fields: no FP64 kind works on them
+    add({LK_F32, LK_F32_1L});
+    if (quad_ok(c, dir, LK_F32_QUAD)) add({LK_F32_QUAD});
+    if (twist_ok(c, dir, LK_F32_TWIST)) add({LK_F32_TWIST});
+  } else {
+    // the filter acts on the FP64 state with an FP64 right-hand side in every
+    // kind: the FP64 eliminations compete with the FP32 ones
+    add({LK_F64_TILE_F32_SOLVE, LK_F64_TILE_F32_SOLVE_1L, LK_F64, LK_F64_1L, LK_F64_SPLIT});
+    for (int k : {LK_F64_TILE_F32_TWIST, LK_F64_TWIST})
+      if (twist_ok(c, dir, k)) add({k});
+    // the streamed filter reads a row of 32 lines per step: coalesced along
+    // eta/zeta only (along xi each lane's row is a line length away)
+    if (dir != 0) add({LK_F64_STREAM_F32});
+  }
+  {  // each kind once, the default first
+    std::vector<int> u;
+    for (int k : kinds)
+      if (std::find(u.begin(), u.end(), k) == u.end()) u.push_back(k);
+    kinds.swap(u);
+  }
+  return kinds;
+}
+
 }  // namespace
 
 // ==================================================================================
@@ -3008,36 +3043,7 @@ int canard_autotune(canard_ctx* c, int32_t reps, double* report, int32_t nmax) {
       for (int dir = 0; dir < 3; ++dir) {
         const int op = grp == 0 ? 1 : 0;
         std::vector<std::pair<int, int>> cand;  // (kind, nc)
-        std::vector<int> kinds{default_kind(c, grp, dir)};
-        if (c->fast()) {  // the one-lane and split FP64 sweeps compete in the fast mode
-          kinds.push_back(LK_F64);
-          kinds.push_back(LK_F64_1L);
-          kinds.push_back(LK_F64_SPLIT);
-        }
-        if (grp != 0 && c->fast() && quad_ok(c, dir, LK_F64_QUAD)) kinds.push_back(LK_F64_QUAD);
-        if (grp != 0 && c->f32() && quad_ok(c, dir, LK_F32_QUAD)) kinds.push_back(LK_F32_QUAD);
-        if (c->f32()) kinds.push_back(grp == 0 ? LK_F64_TILE_F32_SOLVE_1L : LK_F32_1L);
-        if (c->fast() && twist_ok(c, dir, LK_F64_TWIST)) kinds.push_back(LK_F64_TWIST);
-        if (c->f32() && twist_ok(c, dir, LK_F32_TWIST)) kinds.push_back(grp == 0 ? LK_F64_TILE_F32_TWIST : LK_F32_TWIST);
-        // the streamed filter reads a row of 32 lines per step: coalesced along
-        // eta/zeta only (along xi each lane's row is a line length away)
-        if (c->f32() && grp == 0) {
-          if (dir != 0) kinds.push_back(LK_F64_STREAM_F32);
-        } else if (tm_ok(c, dir)) kinds.push_back(LK_F64_TM);
-        // the filter acts on the FP64 state with an FP64 right-hand side in every
-        // kind; the FP64 eliminations (one-lane and split) compete with the FP32 ones there
-        if (c->f32() && grp == 0) {
-          kinds.push_back(LK_F64);
-          kinds.push_back(LK_F64_1L);
-          kinds.push_back(LK_F64_SPLIT);
-          if (twist_ok(c, dir, LK_F64_TWIST)) kinds.push_back(LK_F64_TWIST);
-        }
-        {  // each kind once, the default first
-          std::vector<int> u;
-          for (int k : kinds)
-            if (std::find(u.begin(), u.end(), k) == u.end()) u.push_back(k);
-          kinds.swap(u);
-        }
+        const std::vector<int> kinds = tune_kinds(c, grp, dir);
         for (int k : kinds) {
           cand.push_back({k, 0});
           if (dir != 0 && k != LK_F64_TM && k != LK_F64_STREAM_F32)
@@ -3069,6 +3075,22 @@ int canard_autotune(canard_ctx* c, int32_t reps, double* report, int32_t nmax) {
     rebuild_line_tables(c);
   });
   return rc == CANARD_OK ? rows : -rc;
+}
+
+// The kinds canard_autotune tries for a group and direction, the default first
+// (at most nmax of them); returns their number. Not part of the public header:
+// the check of the candidates.
+int canard_tune_kinds(canard_ctx* c, int32_t group, int32_t dir, int32_t* kinds, int32_t nmax) {
+  if (!c) return -CANARD_ERR_ARG;
+  int n = 0;
+  const int rc = guarded(c, [&] {
+    if (group < 0 || group > 2 || dir < 0 || dir > 2 || nmax < 0 || (nmax > 0 && !kinds))
+      throw ApiError(CANARD_ERR_ARG, "bad line kind argument");
+    const std::vector<int> v = tune_kinds(c, group, dir);
+    n = (int)v.size();
+    std::copy(v.begin(), v.begin() + std::min(n, nmax), kinds);
+  });
+  return rc == CANARD_OK ? n : -rc;
 }
 
 int canard_set_line_kind(canard_ctx* c, int32_t group, int32_t dir, int32_t kind, int32_t chunks) {
