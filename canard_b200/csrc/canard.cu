@@ -1741,12 +1741,12 @@ void build_gcbc_sponge_avg(canard_ctx* c) {
   // GCBC tables need yaco (reference layout) on the host
   std::vector<GcbcTask> gc_tasks;
   std::vector<SpongeTask> sp_tasks;
-  // forced points, GCBC's first, then the sponge's others (ForcedPts)
-  struct Forced { int b; long long l; int n, line[3]; double w[3], sa, sb; bool sp; };
-  std::vector<Forced> gpts;
-  std::vector<int> fb;         // the sponge's other points
-  std::vector<long long> fl;
-  std::vector<double> fsa, fsb;
+  // forced points (ForcedPts): GCBC's, then the sponge's others
+  std::vector<int> gb, gline[3], fb;
+  std::vector<long long> gl, fl;
+  std::vector<double> gw[3], gsa, gsb, fsa, fsb;
+  std::vector<unsigned char> gin;
+  std::vector<std::vector<unsigned char>> mask((size_t)nb);  // BlockDev::forced
   int gc_lines = 0;
   auto partner = [&](int b, int d, int side) -> void* {  // drva of the face that faces (b, d, side)
     for (const FaceLink& L : c->links)
@@ -1771,9 +1771,27 @@ void build_gcbc_sponge_avg(canard_ctx* c) {
     std::vector<int64_t> pts;
     std::vector<double> w;
     gcbc_tables(g, yref.data(), B.gc_faces, pts, w);
-    std::vector<int> at;  // entry of every stored point in gpts, -1: none
-    const size_t g0 = gpts.size();
-    if (!pts.empty()) at.assign((size_t)g.npad, -1);
+    // faces that reach a point, then GCBC's points in memory order (so that
+    // neighbouring entries are neighbouring points): their entries by point, the
+    // others' left unset
+    std::vector<unsigned char>& hits = mask[(size_t)b];
+    std::unique_ptr<int[]> at;
+    if (!pts.empty()) {
+      hits.assign((size_t)g.npad, 0);
+      for (const int64_t l : pts)
+        if (++hits[(size_t)l] > 3)
+          throw ApiError(CANARD_ERR_UNSUPPORTED, "a point within five layers of more than three faces");
+      at.reset(new int[(size_t)g.npad]);
+      for (size_t l = 0; l < hits.size(); ++l)
+        if (hits[l]) {
+          at[l] = (int)gl.size();
+          gl.push_back((long long)l);
+        }
+      const size_t ng = gl.size();
+      gb.resize(ng, b);
+      gsa.resize(ng); gsb.resize(ng); gin.resize(ng);
+      for (int q = 0; q < 3; ++q) { gline[q].resize(ng, -1); gw[q].resize(ng); }
+    }
     for (const GcbcFace& f : B.gc_faces) {
       const int d = f.nn - 1;
       GcbcTask t{};
@@ -1788,15 +1806,11 @@ void build_gcbc_sponge_avg(canard_ctx* c) {
       t.X = g.X; t.Y = g.Y; t.Z = g.Z; t.Xp = g.Xp; t.N = g.ijk[0][d];
       // the face's five layers of points, in face order: at most one face per direction reaches a point
       for (int64_t e = 0; e < (int64_t)5 * t.nbs; ++e) {
-        int& k = at[(size_t)pts[f.first + e]];
-        if (k < 0) {
-          k = (int)gpts.size();
-          gpts.push_back({b, (long long)pts[f.first + e], 0, {-1, -1, -1}, {0, 0, 0}, 0, 0, false});
-        }
-        Forced& q = gpts[k];
-        if (q.n == 3) throw ApiError(CANARD_ERR_UNSUPPORTED, "a point within five layers of more than three faces");
-        q.line[q.n] = gc_lines + (int)(e / 5);
-        q.w[q.n++] = w[f.first + e];
+        const int k = at[(size_t)pts[f.first + e]];
+        int q = 0;
+        while (gline[q][k] >= 0) ++q;
+        gline[q][k] = gc_lines + (int)(e / 5);
+        gw[q][k] = w[f.first + e];
       }
       gc_lines += t.nbs;
       gc_tasks.push_back(t);
@@ -1815,21 +1829,18 @@ void build_gcbc_sponge_avg(canard_ctx* c) {
         SpongeTask st{b, B.sp_pts, B.sp_a, B.sp_b, B.sp_n, 0};
         sp_tasks.push_back(st);
       }
+      if (!sp.empty() && hits.empty()) hits.assign((size_t)g.npad, 0);
       for (size_t e = 0; e < sp.size(); ++e) {
-        const int k = at.empty() ? -1 : at[(size_t)sp[e]];
-        if (k >= 0) {
-          gpts[k].sp = true; gpts[k].sa = a[e]; gpts[k].sb = bb[e];
+        unsigned char& h = hits[(size_t)sp[e]];
+        if (h && at) {
+          const int k = at[(size_t)sp[e]];
+          gin[k] = 1; gsa[k] = a[e]; gsb[k] = bb[e];
         } else {
+          h = 1;
           fb.push_back(b); fl.push_back((long long)sp[e]); fsa.push_back(a[e]); fsb.push_back(bb[e]);
         }
       }
     }
-    // neighbouring entries at neighbouring points (the sponge's are)
-    std::vector<Forced> sorted;
-    sorted.reserve(gpts.size() - g0);
-    for (const int k : at)
-      if (k >= 0) sorted.push_back(gpts[k]);
-    std::copy(sorted.begin(), sorted.end(), gpts.begin() + g0);
   }
   const size_t es = c->f32() ? sizeof(float) : sizeof(double);
   c->gc_dh = dalloc<char>((size_t)5 * gc_lines * es, c->st);
@@ -1842,36 +1853,27 @@ void build_gcbc_sponge_avg(canard_ctx* c) {
   }
   c->gcbc = make_lines_table(c, gc_tasks, false, &GcbcTask::nbs, &GcbcTask::line0);
   c->sponge = make_lines_table(c, sp_tasks, false, &SpongeTask::count, &SpongeTask::first);
-  if (!gpts.empty() || !fb.empty()) {
-    const size_t ng = gpts.size();
-    std::vector<int> pb(ng), ln(3 * ng);
-    std::vector<long long> pl(ng);
-    std::vector<double> sa(ng), sb(ng), pw(3 * ng);
-    std::vector<unsigned char> inside(ng);
-    std::vector<std::vector<unsigned char>> mask((size_t)nb);
-    for (int b = 0; b < nb; ++b) mask[(size_t)b].assign((size_t)c->blocks[b].g.npad, 0);
-    for (size_t e = 0; e < ng; ++e) {
-      const Forced& q = gpts[e];
-      pb[e] = q.b; pl[e] = q.l; sa[e] = q.sa; sb[e] = q.sb;
-      inside[e] = q.sp ? 1 : 0;
-      for (int k = 0; k < 3; ++k) { ln[k * ng + e] = q.line[k]; pw[k * ng + e] = q.w[k]; }
-    }
-    pb.insert(pb.end(), fb.begin(), fb.end());
-    pl.insert(pl.end(), fl.begin(), fl.end());
-    sa.insert(sa.end(), fsa.begin(), fsa.end());
-    sb.insert(sb.end(), fsb.begin(), fsb.end());
-    for (size_t e = 0; e < pb.size(); ++e) mask[(size_t)pb[e]][(size_t)pl[e]] = 1;
+  if (!gl.empty() || !fl.empty()) {
     ForcedPts& F = c->forced;
-    F.b = dupload(pb, c->st); F.l = dupload(pl, c->st);
-    F.sa = dupload(sa, c->st); F.sb = dupload(sb, c->st);
-    F.line = dupload(ln, c->st); F.w = dupload(pw, c->st);
-    F.sponge = dupload(inside, c->st);
-    F.ng = (int)ng; F.ns = (int)fb.size();
+    F.ng = (int)gl.size(); F.ns = (int)fl.size();
+    gb.insert(gb.end(), fb.begin(), fb.end());
+    gl.insert(gl.end(), fl.begin(), fl.end());
+    gsa.insert(gsa.end(), fsa.begin(), fsa.end());
+    gsb.insert(gsb.end(), fsb.begin(), fsb.end());
+    for (int q = 1; q < 3; ++q) {
+      gline[0].insert(gline[0].end(), gline[q].begin(), gline[q].end());
+      gw[0].insert(gw[0].end(), gw[q].begin(), gw[q].end());
+    }
+    F.b = dupload(gb, c->st); F.l = dupload(gl, c->st);
+    F.sa = dupload(gsa, c->st); F.sb = dupload(gsb, c->st);
+    F.line = dupload(gline[0], c->st); F.w = dupload(gw[0], c->st);
+    F.sponge = dupload(gin, c->st);
     std::vector<BlockDev> bdv;
     for (int b = 0; b < nb; ++b) {
-      c->blocks[b].forced = dupload(mask[(size_t)b], c->st);
-      c->blocks[b].dev.forced = c->blocks[b].forced;
-      bdv.push_back(c->blocks[b].dev);
+      BlockState& B = c->blocks[b];
+      if (!mask[(size_t)b].empty()) B.forced = dupload(mask[(size_t)b], c->st);
+      B.dev.forced = B.forced;
+      bdv.push_back(B.dev);
     }
     CK(cudaMemcpyAsync(c->dbd, bdv.data(), bdv.size() * sizeof(BlockDev), cudaMemcpyHostToDevice, c->st));
     CK(cudaStreamSynchronize(c->st));
@@ -1915,24 +1917,19 @@ void build_gcbc_sponge_avg(canard_ctx* c) {
     c->wall_tl = dupload(wl, c->st);
     c->wall_tk = dupload(wk, c->st);
   }
-  // every block-face point
-  {
-    std::vector<int> fb;
-    std::vector<long long> fl;
+  // every block-face point (k_rk_faces, mixed precision)
+  if (c->f32()) {
+    std::vector<int> fpb;
+    std::vector<long long> fpl;
     for (int b = 0; b < nb; ++b) {
       const BlockGeom& g = c->blocks[b].g;
-      for (int z = 0; z < g.Z; ++z)
-        for (int y = 0; y < g.Y; ++y)
-          for (int x = 0; x < g.X; ++x)
-            if (x == 0 || x == g.X - 1 || y == 0 || y == g.Y - 1 || z == 0 || z == g.Z - 1) {
-              fb.push_back(b);
-              fl.push_back((long long)g.dev(x, y, z));
-            }
+      g.for_surface([&](int64_t l) { fpl.push_back((long long)l); });
+      fpb.resize(fpl.size(), b);
     }
-    c->face_n = (int)fb.size();
+    c->face_n = (int)fpl.size();
     if (c->face_n) {
-      c->face_tb = dupload(fb, c->st);
-      c->face_tl = dupload(fl, c->st);
+      c->face_tb = dupload(fpb, c->st);
+      c->face_tl = dupload(fpl, c->st);
     }
   }
   build_average(c, average_tables(geoms, P, Lp, Sf, wall));

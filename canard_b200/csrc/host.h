@@ -49,6 +49,38 @@ struct BlockGeom {
     else { x = j; y = k; z = pos; }
   }
   int64_t ref_index(int x, int y, int z) const { return ((int64_t)z * Y + y) * X + x; }
+  void xyz_of(int64_t l, int& x, int& y, int& z) const {  // of a device index
+    if (npad <= (int64_t)UINT32_MAX) {  // most blocks: 32-bit divisions, several times cheaper
+      const uint32_t u = (uint32_t)l, r = u / (uint32_t)Xp;
+      x = (int)(u - r * (uint32_t)Xp); y = (int)(r % (uint32_t)Y); z = (int)(r / (uint32_t)Y);
+    } else {
+      const int64_t r = l / Xp;
+      x = (int)(l - r * Xp); y = (int)(r % Y); z = (int)(r / Y);
+    }
+  }
+  // the block's surface points, numbered in memory order
+  int64_t ring() const { return 2 * (int64_t)X + 2 * (Y - 2); }  // of a z plane between the ends
+  int64_t nsurf() const { return 2 * (int64_t)X * Y + (Z - 2) * ring(); }
+  bool on_surface(int x, int y, int z) const {
+    return x == 0 || x == X - 1 || y == 0 || y == Y - 1 || z == 0 || z == Z - 1;
+  }
+  int64_t surf(int x, int y, int z) const {
+    if (z == 0) return (int64_t)y * X + x;
+    const int64_t base = (int64_t)X * Y + (z - 1) * ring();
+    if (z == Z - 1) return base + (int64_t)y * X + x;
+    if (y == 0) return base + x;
+    if (y == Y - 1) return base + X + 2 * (int64_t)(Y - 2) + x;
+    return base + X + 2 * (int64_t)(y - 1) + (x != 0);
+  }
+  template <class F>
+  void for_surface(F&& f) const {  // f(device index), in memory order
+    for (int z = 0; z < Z; ++z)
+      for (int y = 0; y < Y; ++y) {
+        if (z == 0 || z == Z - 1 || y == 0 || y == Y - 1)
+          for (int x = 0; x < X; ++x) f(dev(x, y, z));
+        else { f(dev(0, y, z)); f(dev(X - 1, y, z)); }
+      }
+  }
 };
 
 void make_geom(const canard_block_desc& d, int case_id, int bic, BlockGeom& g);

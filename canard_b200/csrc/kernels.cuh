@@ -70,8 +70,8 @@ struct BlockDev {
   // FP64: state, metric and Jacobian masters, and the FP64 work fields
   double *qa, *qo, *de, *p, *mu, *xim, *etm, *zem, *yaco, *tau, *scr, *xyz;
   Work<float> f;  // FP32 work fields and metric copies (mixed precision only)
-  // 1 at the points whose right-hand side the GCBC or the sponge changes (null:
-  // none in the block); one byte per stored point
+  // not 0 at the points whose right-hand side the GCBC or the sponge changes
+  // (null: none in the block); one byte per stored point
   const unsigned char* forced;
   double* qb;  // time-averaged recording (5 fields), while it is on
 };
