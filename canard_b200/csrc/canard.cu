@@ -1050,7 +1050,9 @@ Table<FaceTask> make_face_table(canard_ctx* c, std::vector<FaceTask> v, bool tra
   for (auto& t : v) { t.line0 = tot; first.push_back(tot); tot += t.nbs; T.most = std::max(T.most, t.nbs); }
   T.ntasks = (int)v.size();
   T.total = tot;
-  T.bytes = (double)tot * (12 + (v.empty() ? 0 : (v[0].nt ? 3 : 2))) * (kind ? sizeof(float) : sizeof(double));
+  // a face that is not exchanged reads one value and advances its chain
+  for (const auto& t : v)
+    T.bytes += (double)t.nbs * (t.exch ? 12 + (t.nt ? 3 : 2) : 3) * (kind ? sizeof(float) : sizeof(double));
   T.tasks = dupload(v, c->st);
   T.first = dupload(first, c->st);
   if (transient) { c->transient.push_back(T.tasks); c->transient.push_back(T.first); }
