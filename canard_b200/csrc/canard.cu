@@ -68,7 +68,7 @@ const int kNnf[3] = {2, 3, 1};  // filter direction order (src/mo_numerics.f90:2
 template <class T>
 struct Table {
   T* tasks = nullptr;
-  int* first = nullptr;  // line tables: the task of every tile; others: each task's first line
+  int* first = nullptr;  // line tables: the task of every tile; GCBC, sponge: each task's first line
   int ntasks = 0;
   int total = 0;  // tiles or lines
   size_t smem = 0;
@@ -79,7 +79,6 @@ struct Table {
   int most = 0;  // face tables: lines of the largest face
 };
 
-// Element types of a line launch: tile (field) type and elimination type.
 // Element types and solve form of a line launch: FP64 one-lane sweeps
 // (bit-exact); FP32 fields; FP64 fields with an FP32 elimination. The FP32
 // eliminations come as the split solve (16 lines per tile) or the one-lane
@@ -538,8 +537,9 @@ void chunking(int L, int& nc, int& cr, int nc_req = 0) {
   if (nc == 1) cr = (L + 1) / 2 * 2;
 }
 
-// xi lines (dir 0) move as one bulk copy per line: per-lane copy instructions
-// are costly enough that chunking them does not pay.
+// xi lines (dir 0) are not chunked: they move as one bulk copy per line (per-lane
+// copy instructions are costly enough that chunking them does not pay) or, in
+// the one-lane sweeps, as tensor boxes (one_lane_tile).
 void chunking_dir(int dir, int L, int& nc, int& cr, int nc_req = 0) {
   if (dir == 0) {
     nc = 1;
@@ -1008,7 +1008,6 @@ template <class ColFn>
 std::vector<FaceTask> face_tasks(const canard_ctx* c, int nt, int n45, int m, int exch_dir, ColFn col,
                                  int only_case = -1, bool f32 = false, bool skip_selfp = false) {
   std::vector<FaceTask> out;
-  int line0 = 0;
   for (const FaceLink& L : c->links) {
     if (only_case >= 0 && c->blocks[L.src_b].g.case_id != only_case) continue;
     const BlockState& S = c->blocks[L.src_b];
@@ -1035,8 +1034,6 @@ std::vector<FaceTask> face_tasks(const canard_ctx* c, int nt, int n45, int m, in
     t.XA = R.g.X; t.YA = R.g.Y; t.ZA = R.g.Z; t.XpA = R.g.Xp; t.NA = R.g.ijk[0][d];
     t.nbs = S.g.nbs[d];
     t.nj = S.g.ijk[1][d] + 1;
-    t.line0 = line0;
-    line0 += t.nbs;
     out.push_back(t);
   }
   return out;
@@ -1045,17 +1042,13 @@ std::vector<FaceTask> face_tasks(const canard_ctx* c, int nt, int n45, int m, in
 Table<FaceTask> make_face_table(canard_ctx* c, std::vector<FaceTask> v, bool transient, int kind = 0) {
   Table<FaceTask> T;
   T.kind = kind;
-  std::vector<int> first;
-  int tot = 0;
-  for (auto& t : v) { t.line0 = tot; first.push_back(tot); tot += t.nbs; T.most = std::max(T.most, t.nbs); }
+  for (const auto& t : v) { T.total += t.nbs; T.most = std::max(T.most, t.nbs); }
   T.ntasks = (int)v.size();
-  T.total = tot;
   // a face that is not exchanged reads one value and advances its chain
   for (const auto& t : v)
     T.bytes += (double)t.nbs * (t.exch ? 12 + (t.nt ? 3 : 2) : 3) * (kind ? sizeof(float) : sizeof(double));
   T.tasks = dupload(v, c->st);
-  T.first = dupload(first, c->st);
-  if (transient) { c->transient.push_back(T.tasks); c->transient.push_back(T.first); }
+  if (transient) c->transient.push_back(T.tasks);
   return T;
 }
 
@@ -2925,9 +2918,9 @@ int canard_mpigo(canard_ctx* c, const double* const* fields, int32_t ncols, int3
   });
 }
 
-// One field through one line solve; in a mixed-precision context the
-// derivative runs on an FP32 copy and the filter on the FP64 field with an
-// FP32 elimination, as on the step path.
+// One field through one line solve, in a mixed-precision context the derivative
+// on an FP32 copy and the filter on the FP64 field with an FP32 elimination. One
+// kind per precision, whatever the line length and the tuning of the step.
 static void unit_line(canard_ctx* c, int iblock, const double* in, double* out, int dir, int nt, int m) {
   const int b = block_index(c, 0, iblock);
   BlockState& B = c->blocks[b];
@@ -3197,7 +3190,6 @@ constexpr int kNaMaxPoints = 1024;   // points per line the scratch's factor tab
                                      // tile allows fewer: 906 along xi, 896 along eta or zeta)
 constexpr size_t kNaTask = 0;        // LineTask
 constexpr size_t kNaFace = 512;      // up to 2 FaceTask
-constexpr size_t kNaIdx = 1536;      // (unused int), line0 of the 2 face tasks
 constexpr size_t kNaErr = 1600;      // device error flag
 constexpr size_t kNaChain = 1608;    // unused third send component (2 doubles)
 constexpr size_t kNaMaps = 1664;     // 2 CUtensorMap, 64-byte aligned
@@ -3210,7 +3202,7 @@ constexpr int kNaMaxTiles = 8192;
 constexpr size_t kNaTiles = kNaRecv + (size_t)4 * kNaMaxLines * sizeof(double);
 constexpr size_t kNaBytes = kNaTiles + (size_t)kNaMaxTiles * sizeof(int);
 static_assert(sizeof(LineTask) <= kNaFace - kNaTask, "LineTask slot");
-static_assert(2 * sizeof(FaceTask) <= kNaIdx - kNaFace, "FaceTask slots");
+static_assert(2 * sizeof(FaceTask) <= kNaErr - kNaFace, "FaceTask slots");
 static_assert(sizeof(DevScheme) <= kNaLu - kNaScheme, "scheme slot");
 static_assert(kNaMaps % 64 == 0 && kNaLu % 256 == 0 && kNaRecv % 256 == 0, "alignment");
 }  // namespace
@@ -3334,7 +3326,7 @@ extern "C" int canard_deriv_noalloc(const double* d_in, double* d_out, int32_t l
         q.nn = nn; q.sb = sb; q.nt = 0; q.exch = 1; q.corr = 0; q.iik = 1; q.ra0k = 0.0;
         q.X = g.X; q.Y = g.Y; q.Z = g.Z; q.Xp = g.Xp; q.N = L - 1;
         q.XA = g.X; q.YA = g.Y; q.ZA = g.Z; q.XpA = g.Xp; q.NA = L - 1;
-        q.nbs = nbs; q.nj = g.ijk[1][dir] + 1; q.line0 = nf * nbs;
+        q.nbs = nbs; q.nj = g.ijk[1][dir] + 1;
         ++nf;
       }
     }
@@ -3352,10 +3344,8 @@ extern "C" int canard_deriv_noalloc(const double* d_in, double* d_out, int32_t l
       maps[0] = field_map(d_in, g.X, g.Y, g.Z, g.Xp, dir, t.by);
       maps[1] = field_map(d_out, g.X, g.Y, g.Z, g.Xp, dir, t.by);
     }
-    const int idx[3] = {0, 0, nbs};
     CK(cudaMemcpyToSymbolAsync(g_noalloc_scratch, &t, sizeof(t), kNaTask, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyToSymbolAsync(g_noalloc_scratch, f, sizeof(f), kNaFace, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyToSymbolAsync(g_noalloc_scratch, idx, sizeof(idx), kNaIdx, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyToSymbolAsync(g_noalloc_scratch, maps, sizeof(maps), kNaMaps, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyToSymbolAsync(g_noalloc_scratch, &ds, sizeof(ds), kNaScheme, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyToSymbolAsync(g_noalloc_scratch, lu.data(), lu.size() * sizeof(double), kNaLu,

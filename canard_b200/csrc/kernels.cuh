@@ -109,7 +109,7 @@ struct LineTask {
   int tile0, ntiles, ntx;  // first global tile, tiles, x-tiles per row (dir 2/3)
   int nbox, by;            // chunks per tile and positions per chunk
   // one-lane sweeps: staged factor rows; xi tiles: line pitch, and whether a
-  // tile moves as one tensor box
+  // tile moves as tensor boxes (nbox of them)
   int ts, pitch, xt;
 };
 
@@ -126,7 +126,7 @@ struct FaceTask {
   double ra0k;
   int X, Y, Z, Xp, N;       // sender geometry
   int XA, YA, ZA, XpA, NA;  // receiver geometry
-  int nbs, nj, line0;
+  int nbs, nj;
 };
 
 struct GcbcTask {  // one GCBC face of one block
@@ -370,15 +370,6 @@ struct B8 {
     for (int k = 0; k < 8; ++k) { u1[k] = cf.U1(i - k); u2[k] = cf.U2(i - k); u3[k] = cf.U3(i - k); }
   }
 };
-template <class TT>
-struct O8 {
-  TT o[8];
-  __device__ __forceinline__ void load(const TT* __restrict__ og, int ogs, int i) {
-#pragma unroll
-    for (int k = 0; k < 8; ++k) o[k] = __ldg(og + (long long)(i - k) * ogs);
-  }
-};
-
 // Right-hand sides of the derivative's rows i..i+7 (reads rows up to i+9);
 // window w0..w3 = s[i-2..i+1] on entry, s[i+6..i+9] on return
 template <int ST, class TT>
@@ -407,22 +398,6 @@ __device__ __forceinline__ void chain8_fwd(TT* __restrict__ s, int i, const F8<R
   am2 = a[6]; am1 = a[7];
 }
 
-// forward rows i..i+7 of the derivative; window w0..w3 = s[i-2..i+1]
-template <int ST, class TT, class RS>
-__device__ __forceinline__ void fwd8_deriv_c(TT* __restrict__ s, int i, const F8<RS>& f, TT& w0, TT& w1, TT& w2,
-                                             TT& w3, RS& am2, RS& am1) {
-  TT r[8];
-  rhs8_deriv<ST, TT>(s, i, w0, w1, w2, w3, r);
-  chain8_fwd<ST, TT, RS>(s, i, f, r, am2, am1);
-}
-template <int ST, class TT, class RS, class CF>
-__device__ __forceinline__ void fwd8_deriv(TT* __restrict__ s, int i, const CF& cf, TT& w0, TT& w1, TT& w2, TT& w3,
-                                           RS& am2, RS& am1) {
-  F8<RS> f;
-  f.load(cf, i);
-  fwd8_deriv_c<ST, TT, RS>(s, i, f, w0, w1, w2, w3, am2, am1);
-}
-
 // Right-hand sides of the filter's rows i..i+7 (reads rows up to i+10);
 // window w0..w5 = s[i-3..i+2] on entry, s[i+5..i+10] on return
 // DIRECT: the right-hand side of the filtered values themselves, (B x)_i =
@@ -444,57 +419,25 @@ __device__ __forceinline__ void rhs8_filter(const TT* __restrict__ s, int i, TT 
   w0 = win[8]; w1 = win[9]; w2 = win[10]; w3 = win[11]; w4 = win[12]; w5 = win[13];
 }
 
-// forward rows i..i+7 of the filter; window w0..w5 = s[i-3..i+2]
-template <int ST, class TT, class RS>
-__device__ __forceinline__ void fwd8_filter_c(TT* __restrict__ s, int i, const F8<RS>& f, TT fa, TT fb, TT fc,
-                                              TT& w0, TT& w1, TT& w2, TT& w3, TT& w4, TT& w5, RS& am2, RS& am1) {
-  TT r[8];
-  rhs8_filter<ST, TT>(s, i, fa, fb, fc, w0, w1, w2, w3, w4, w5, r);
-  chain8_fwd<ST, TT, RS>(s, i, f, r, am2, am1);
-}
-template <int ST, class TT, class RS, class CF>
-__device__ __forceinline__ void fwd8_filter(TT* __restrict__ s, int i, const CF& cf, TT fa, TT fb, TT fc, TT& w0,
-                                            TT& w1, TT& w2, TT& w3, TT& w4, TT& w5, RS& am2, RS& am1) {
-  F8<RS> f;
-  f.load(cf, i);
-  fwd8_filter_c<ST, TT, RS>(s, i, f, fa, fb, fc, w0, w1, w2, w3, w4, w5, am2, am1);
-}
-
-// back substitution rows i, i-1, ..., i-7. ADD (filter): each row is stored
-// as original + increment, the originals in o.
+// back substitution rows i, i-1, ..., i-7
 template <int ST, class TT, class RS>
 __device__ __forceinline__ void bwd_p8(const TT* __restrict__ s, int i, const B8<RS>& b, RS (&p)[8]) {
 #pragma unroll
   for (int k = 0; k < 8; ++k) p[k] = b.u1[k] * RS(s[(i - k) * ST]);
 }
-template <int ST, class TT, class RS, int ADD>
-__device__ __forceinline__ void bwd_chain8(TT* __restrict__ s, int i, const B8<RS>& b, const RS (&p)[8],
-                                           const O8<TT>& o, RS& cp1, RS& cp2) {
+template <int ST, class TT, class RS>
+__device__ __forceinline__ void bwd_chain8(TT* __restrict__ s, int i, const B8<RS>& b, const RS (&p)[8], RS& cp1,
+                                           RS& cp2) {
   RS c[8];
   c[0] = (p[0] - b.u2[0] * cp1) - b.u3[0] * cp2;
   c[1] = (p[1] - b.u2[1] * c[0]) - b.u3[1] * cp1;
 #pragma unroll
   for (int k = 2; k < 8; ++k) c[k] = (p[k] - b.u2[k] * c[k - 1]) - b.u3[k] * c[k - 2];
 #pragma unroll
-  for (int k = 0; k < 8; ++k) s[(i - k) * ST] = ADD ? o.o[k] + TT(c[k]) : TT(c[k]);
+  for (int k = 0; k < 8; ++k) s[(i - k) * ST] = TT(c[k]);
   cp2 = c[6];
   cp1 = c[7];
 }
-template <int ST, class TT, class RS, int ADD>
-__device__ __forceinline__ void bwd8_c(TT* __restrict__ s, int i, const B8<RS>& b, const O8<TT>& o, RS& cp1,
-                                       RS& cp2) {
-  RS p[8];
-  bwd_p8<ST, TT, RS>(s, i, b, p);
-  bwd_chain8<ST, TT, RS, ADD>(s, i, b, p, o, cp1, cp2);
-}
-template <int ST, class TT, class RS, class CF>
-__device__ __forceinline__ void bwd8(TT* __restrict__ s, int i, const CF& cf, RS& cp1, RS& cp2) {
-  B8<RS> b;
-  b.load(cf, i);
-  O8<TT> o;
-  bwd8_c<ST, TT, RS, 0>(s, i, b, o, cp1, cp2);
-}
-
 // The task of this CTA's tile: tdiv > 0 when every task of the launch has
 // tdiv tiles (no table read on the CTA's start-up path), else the table.
 __device__ __forceinline__ int tile_of(const int* __restrict__ tile_task, int tdiv) {
@@ -644,7 +587,6 @@ __device__ __forceinline__ void bwd_rows(TT* s, int ihi, int ilo, const CF& cf, 
   int i = ihi;
   if (i - 7 >= ilo) {
     B8<RS> bn;
-    O8<TT> on;
     RS pn[8];
     bn.load(cf, i);
     bwd_p8<ST, TT, RS>(s, i, bn, pn);
@@ -655,10 +597,10 @@ __device__ __forceinline__ void bwd_rows(TT* s, int ihi, int ilo, const CF& cf, 
       for (int k = 0; k < 8; ++k) pu[k] = pn[k];
       bn.load(cf, i - 8);
       bwd_p8<ST, TT, RS>(s, i - 8, bn, pn);
-      bwd_chain8<ST, TT, RS, 0>(s, i, bu, pu, on, cp1, cp2);
+      bwd_chain8<ST, TT, RS>(s, i, bu, pu, cp1, cp2);
       i -= 8;
     }
-    bwd_chain8<ST, TT, RS, 0>(s, i, bn, pn, on, cp1, cp2);
+    bwd_chain8<ST, TT, RS>(s, i, bn, pn, cp1, cp2);
     i -= 8;
   }
   for (; i >= ilo; --i) {

@@ -553,10 +553,11 @@ constexpr int kLineSlack = 32;  // a row-major tile's reads may touch one row pa
 // units with contraction; the FP64 filter then solves for the filtered values.
 // Eta/zeta tiles are [row][32 lines] and move in chunks (loads overlap the
 // forward sweep, stores the back substitution); xi tiles are one or two
-// [line][pitch] boxes (T.xt, lines of up to 508 FP64 points) or, for longer
-// lines, one bulk copy per line: 32 bulk copies cost a CTA 3.0 thousand cycles
-// to issue and 32 bulk stores 5.6 thousand, a box 1.4 thousand with its task's
-// start-up.
+// [line][pitch] boxes (T.xt, lines of up to 508 FP64 or 504 FP32 points; one box,
+// up to 254 points, for a filter that solves for the increment, whose store is
+// one add per line) or, for longer lines, one bulk copy per line: 32 bulk copies
+// cost a CTA 3.0 thousand cycles to issue and 32 bulk stores 5.6 thousand, a box
+// 1.4 thousand with its task's start-up.
 //
 // A filter that solves for the increment adds the originals row by row along
 // eta and zeta; along xi the tile keeps the increment and one bulk FP64

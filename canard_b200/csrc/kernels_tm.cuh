@@ -319,7 +319,7 @@ __device__ __forceinline__ void tm_backward(const LuRows<double>& F, int N, uint
   }
 }
 
-// Derivative forward sweep (sweep_deriv's rows); returns a(N), a(N-1).
+// Derivative forward sweep (sweep_line's rows); returns a(N), a(N-1).
 template <int DIR>
 __device__ __forceinline__ bool tm_forward_deriv(TmStream<DIR>& R, const LuRows<double>& F, int ndf0, int ndf1,
                                                  const DevScheme* __restrict__ sc, double r00, double r10,
@@ -402,7 +402,7 @@ __device__ __forceinline__ bool tm_forward_deriv(TmStream<DIR>& R, const LuRows<
   return R.ok;
 }
 
-// Filter forward sweep (sweep_filter's rows); returns a(N), a(N-1).
+// Filter forward sweep (sweep_line's rows); returns a(N), a(N-1).
 template <int DIR>
 __device__ __forceinline__ bool tm_forward_filter(TmStream<DIR>& R, const LuRows<double>& F, int ndf0, int ndf1,
                                                   const DevScheme* __restrict__ sc, double r00, double r10,
