@@ -52,3 +52,14 @@ def test_fast_along_zeta(op, periodic):
 def test_fp32_along_eta(periodic):
     for L in ETA:
         check(2, L, api.FP32_MIXED, "fp32-one-lane", 0, 5e-6, periodic)
+
+
+@pytest.mark.parametrize("periodic", [True, False])
+def test_longest_lines(periodic):
+    """Lines whose tile leaves the CTA's shared memory no room, or little, for staged factors."""
+    for nn, L in ((1, 905), (1, 906), (2, 895), (2, 896), (3, 896)):
+        for op in (0, 1):
+            check(nn, L, api.FP64, "fp64", op, 0, periodic)
+            check(nn, L, api.FP64_FAST, "fp64-one-lane", op, 1e-13, periodic)
+    for nn, L in ((1, 1800), (1, 1801), (2, 1801), (3, 1801)):
+        check(nn, L, api.FP32_MIXED, "fp32-one-lane", 0, 5e-6, periodic)
