@@ -275,7 +275,7 @@ def workload_cases(args, cases, world=1, rank=0):
 def config_dict(args, workload, ncases, job_points, npts, world):
     """The bench line's config, the same for the device arm and the reference arm."""
     mode = {"fp64": "FP64, bit-exact with the reference's operation order",
-            "fast": "FP64 fast mode (split and two-ended line solves with FMA; within 1e-10 of the reference "
+            "fast": "FP64 fast mode (one-lane and two-ended line solves with FMA; within 1e-10 of the reference "
                     "after 10 steps)",
             "fp32": "FP32-mixed (FP32 line solves and fluxes; FP64 state, RK update, metrics and LU)"}[args.precision]
     return {"workload": workload, "cases": ncases, "points": job_points, "precision": args.precision,
@@ -375,7 +375,8 @@ def kernels_mode(args, api, cases, torch):
     # right-hand sides (an autotuner candidate), pinned for the comparison
     for prec, name in ((api.FP64, "fp64"), (api.FP64, "fp64-tmem"), (api.FP64_FAST, "fp64-fast"),
                        (api.FP64_FAST, "fp64-quad"), (api.FP32_MIXED, "fp32"), (api.FP32_MIXED, "fp32-quad"),
-                       (api.FP32_MIXED, "fp32-stream"), (api.FP64_FAST, "fp64-twist"), (api.FP32_MIXED, "fp32-twist")):
+                       (api.FP32_MIXED, "fp32-stream"), (api.FP64_FAST, "fp64-twist"), (api.FP32_MIXED, "fp32-twist"),
+                       (api.FP64_FAST, "fp64-one-lane"), (api.FP64_FAST, "fp64-split"), (api.FP32_MIXED, "fp32-split")):
         ctx = api.Context(cs, precision=prec, setup=False, upload_state=False)
         for op in (0, 1):
             if (name == "fp32-stream" and op == 0) or (name.endswith("quad") and op == 1):
@@ -390,12 +391,15 @@ def kernels_mode(args, api, cases, torch):
                 if name.endswith("twist"):  # two-ended solve (two warps per 32 lines)
                     kt = name if (op == 0 or name == "fp64-twist") else "fp64-tile/fp32-twist"
                     ctx.set_line_kind("flux" if op == 0 else "filter", "xi eta zeta".split()[nn - 1], kt)
+                if name in ("fp64-one-lane", "fp64-split", "fp32-split"):
+                    kt = name if op == 0 or name != "fp32-split" else "fp64-tile/fp32-split"
+                    ctx.set_line_kind("flux" if op == 0 else "filter", "xi eta zeta".split()[nn - 1], kt)
                 # xi runs on the shared-memory tiles here too: the filter's interface calls
                 # advance the send chains of all directions in the oracle's order
                 out, ms = ctx.line_bench(op, nn, fields, reps=args.steps)
                 if name == "fp64-tmem" and nn == 1:
                     continue
-                es = 4 if (name in ("fp32", "fp32-quad", "fp32-twist") and op == 0) else 8
+                es = 4 if (name in ("fp32", "fp32-quad", "fp32-twist", "fp32-split") and op == 0) else 8
                 gbs = 5 * blk.npts * 2 * es / (ms / 1e3) / 1e9
                 r = ref[(op, nn)]
                 err = float(np.linalg.norm((out - r).ravel()) / np.linalg.norm(r.ravel()))

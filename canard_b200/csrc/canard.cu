@@ -1168,10 +1168,12 @@ bool any_viscous(const canard_ctx* c) {
 }
 
 // Three launches of at most this many tiles gain from running side by side
-// (about one wave each: 20 steps of TGV 64, 780 tiles a launch, 16.7 -> 15.6 ms);
-// larger ones take each other's cache lines (six 101 x 101 x 17 blocks, up to
-// 9700 tiles a launch, 41.2 ms in order and 42.4 side by side; four 193 x 129 x
-// 65 blocks 160.4 and 161.6).
+// (about one wave each), larger ones take each other's cache lines. In order /
+// side by side, us a step, by the tiles of a flux launch: TGV 48^3 (490) 437 / 391,
+// 64^3 (975) 635 / 589, mixed 365 / 315, 80^3 (1215) 907 / 893, mixed 565 / 485, 96^3
+// (1940) 1380 / 1383, fast 1204 / 1197, mixed 800 / 746, 104^3 (2100) 1595 / 1615, mixed
+// 958 / 869; above the limit 144^3 plain 3424 / 3444, mixed 1956 / 1906, six 101 x 101
+// x 17 blocks 1810 / 1861, four 97 x 65 x 33 blocks 1448 / 1533.
 bool few_tiles(const Table<LineTask> (&T)[3]) {
   int most = 0;
   for (const auto& t : T) most = std::max(most, t.total);

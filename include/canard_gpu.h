@@ -46,7 +46,7 @@ extern "C" {
 
 #define CANARD_FP64 0            /* plain FP64 path, bit-identical to the reference's operation order */
 #define CANARD_FP32_MIXED 1      /* FP32 line solves/fluxes, FP64 state, RK, metrics, LU */
-#define CANARD_FP64_FAST 2       /* FP64 throughout, line solves split in two halves per line with FMA,
+#define CANARD_FP64_FAST 2       /* FP64 throughout, line solves with FMA (long lines from both ends),
                                     the filter direction by direction over the five fields: not
                                     bit-identical, rounding-level differences (<= 1e-10 relative L2
                                     after 10 steps is the bound its tests hold) */
@@ -283,9 +283,9 @@ int canard_version(void);
  * of the direction's derivative (op 0) or filter (op 1, in place) over all of
  * them runs after their interface contraction and its result is copied to
  * out; then `reps` more launches are timed with CUDA events on the context
- * stream and *ms_per_launch receives their average. In a mixed-precision
- * context the derivative runs on FP32 copies, the filter on the FP64 fields
- * with an FP32 elimination, as on the step path. */
+ * stream and *ms_per_launch receives their average. The line kernel is the
+ * step path's (the default or a pinned kind): in a mixed-precision context the
+ * derivative runs on FP32 copies, the filter on the FP64 fields. */
 int canard_line_bench(canard_ctx* ctx, int32_t op, int32_t nn, int32_t nfields, const double* in, double* out,
                       int32_t reps, double* ms_per_launch);
 
@@ -300,8 +300,9 @@ int canard_line_bench(canard_ctx* ctx, int32_t op, int32_t nn, int32_t nfields, 
  * lines per tile), and for the filter, which filters the FP64 state with an
  * FP64 right-hand side in every kind, the FP64 eliminations (one-lane and
  * split) as well; fast FP64 contexts try the split FP64 solve and the one-lane
- * FP64 sweeps, with and without FMA. Where every block's lines along the direction have at
- * least 32 points, the two-ended solves (kinds 10-12) compete too. The
+ * FP64 sweeps, with and without FMA. Where every block's lines along the
+ * direction have at least 32 points, the two-ended solves (kinds 10-12) compete
+ * too. The
  * fastest choice is installed in the step tables. Returns the number of groups
  * (9) and fills up to nmax report rows of 6 doubles: group, direction
  * (0..2), chosen kind, chosen chunk count (0 = default), its ms per launch
@@ -315,8 +316,8 @@ int canard_autotune(canard_ctx* ctx, int32_t reps, double* report, int32_t nmax)
  * FP32 one-lane, 4 FP64 tile / FP32 one-lane, 5 FP64 with the elimination
  * results in tensor memory (eta/zeta, 16..257 points per line), 6 the filter
  * of the FP64 state streamed into FP32 right-hand sides (mixed precision), 7
- * FP64 split solve with FMA (FP64 and fast FP64 contexts), 8 and 9 the derivative's quad split solve (four lanes per line) on
- * FP64 fields (FP64 and fast FP64 contexts) and on FP32 fields (mixed
+ * FP64 split solve with FMA (FP64 and fast FP64 contexts), 8 and 9 the
+ * derivative's quad split solve (four lanes per line) on FP64 fields (FP64 and fast FP64 contexts) and on FP32 fields (mixed
  * precision), for lines of at least about 4 x 60 points (FP64) or 4 x 40
  * (FP32); 10, 11 and 12 the two-ended solve (two warps per tile of 32 lines,
  * one eliminating from each end of the line, the four unknowns where they
