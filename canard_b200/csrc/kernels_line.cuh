@@ -679,8 +679,9 @@ __global__ void __maxnreg__(168) k_line(const LineTask* __restrict__ tasks, cons
   const LineFac<RS> F{fl, bu, lu, RS(T.cl1), RS(T.cl2), RS(T.cu1), RS(T.cu2), RS(T.cu3), TR, T.c0, L - 4, L};
   if (!mbar_wait(bars, 0) || !mbar_wait(bars + NC - 1, 0)) {
     if (lane == 0) atomicExch(err, kErrTimeout);
-    // copies may still be landing: wait for the other chunks (bounded) before exit
-    for (int c = 1; c < NC - 1; ++c) mbar_wait(bars + c, 0);
+    // copies may still be landing: wait for the other chunks, the last among
+    // them where the first gave up (bounded), before exit
+    for (int c = 1; c < NC; ++c) mbar_wait(bars + c, 0);
     return;
   }
   __syncwarp();
